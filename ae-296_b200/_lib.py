@@ -9,7 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from .build import LIB_PATH
+from .build import HOST_PATH, LIB_PATH
 
 F16, BF16, F32 = 0, 1, 2
 MID_ROUND, NO_TENSOR, ONLY_SHRINK, ONLY_EXPAND, DELTA_THEN_ADD, KEEP_PARTIALS = 1, 2, 4, 8, 32, 64
@@ -56,6 +56,8 @@ SYMBOLS = {
     "b200_lora_plan_build": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p, C.c_int32, C.c_int32,
                                        C.POINTER(Adapters), C.c_void_p]),
     "b200_lora_plan_from_segments": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p, C.c_void_p,
+                                               C.c_int32, C.c_int32, C.POINTER(Adapters), C.c_void_p]),
+    "b200_lora_plan_from_requests": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p, C.c_void_p,
                                                C.c_int32, C.c_int32, C.POINTER(Adapters), C.c_void_p]),
     "b200_lora_plan_read": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                       C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.c_void_p]),
@@ -118,6 +120,26 @@ def lib() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _LIB = handle
     return _LIB
+
+
+_HOST = None
+
+
+def host():
+    """The native host path of the ops (``csrc/host.cpp``): the same C ABI, called with the operands read from
+    the tensor objects in C++."""
+    global _HOST
+    if _HOST is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise ImportError(f"{HOST_PATH} is missing: build it with `python -m ae296_b200.build`")
+        import importlib.util
+        import torch                        # noqa: F401  (its libraries must be loaded first)
+        spec = importlib.util.spec_from_file_location("_b200host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _HOST = module
+    return _HOST
 
 
 def check(code: int, what: str = "") -> None:

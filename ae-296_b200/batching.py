@@ -45,10 +45,9 @@ def plan_for_requests(batch: LoraBatch, pool: AdapterPool, lora_ids: torch.Tenso
         if total_token_num != n_req:
             raise ValueError("a decode batch has one token per request")
         return batch.set_ids(lora_ids.contiguous(), pool, tiles=False)
-    starts = torch.empty(n_req + 1, dtype=torch.int32, device=lora_ids.device)
-    starts[:n_req] = b_start_loc
-    starts[n_req] = int(total_token_num)
-    return batch.set_segments(starts, lora_ids.contiguous(), int(total_token_num), pool, tiles=True)
+    # the library takes the start of every request and ends the last one at total_token_num: building a table
+    # with the end in it took a small copy from the host, which waits for everything queued before it
+    return batch.set_segments(b_start_loc.contiguous(), lora_ids.contiguous(), int(total_token_num), pool, tiles=True)
 
 
 def delta_cost_us(ranks_of_requests: Sequence[int], tokens_of_requests: Sequence[int], adapters_of_requests: Sequence[int],

@@ -1,0 +1,390 @@
+// Native host path of the Python ops: from tensors and pool objects to one C-ABI call.
+//
+// A decode step makes 64 to 160 applies, each of a few microseconds on the GPU, so what Python spends per
+// call decides the step's time.  Reading the tensors through ctypes (a data_ptr() call, two stride() calls
+// and a structure field per operand, and a NumPy pass over the ranks) took 35-40 us per fused apply and
+// 21 us per operator call; here the operands are read from the tensor objects directly and the whole call
+// costs about 1 us besides the CUDA launches.
+//
+// The functions take the short path only: operands that are exactly what the ops document.  Anything else
+// (a wrong shape or type, a table that has to grow) returns kSlow and the Python code beside the call
+// raises the error or prepares what is missing.  The GIL is given up around the CUDA calls.
+#include <Python.h>
+
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <mutex>
+#include <vector>
+
+#include "b200_lora.h"
+
+namespace {
+
+constexpr long kSlow = 1;          // "not for the short path" (status codes are <= 0)
+
+// attribute names, interned once
+PyObject *s_wa, *s_wb, *s_h_in, *s_h_out, *s_ranks, *s_scalings, *s_cum_ranks, *s_n_adapters, *s_n_layers, *s_r_pool,
+    *s_packed, *s_ranks_host, *s_cum_host, *s_buf, *s_nbytes, *s_max_tokens, *s_n_tokens;
+
+struct Ref {                       // owned reference
+    PyObject* o;
+    explicit Ref(PyObject* p) : o(p) {}
+    ~Ref() { Py_XDECREF(o); }
+    Ref(const Ref&) = delete;
+    Ref& operator=(const Ref&) = delete;
+    explicit operator bool() const { return o != nullptr; }
+};
+
+bool get_int(PyObject* obj, PyObject* name, int64_t& out) {
+    Ref v(PyObject_GetAttr(obj, name));
+    if (!v) return false;
+    out = PyLong_AsLongLong(v.o);
+    return !(out == -1 && PyErr_Occurred());
+}
+
+// A CUDA tensor attribute; None gives a null pointer when `optional`.
+bool get_ptr(PyObject* obj, PyObject* name, bool optional, const void*& out, at::ScalarType* dtype = nullptr) {
+    Ref v(PyObject_GetAttr(obj, name));
+    if (!v) return false;
+    out = nullptr;
+    if (v.o == Py_None) return optional;
+    if (!THPVariable_Check(v.o)) return false;
+    const at::Tensor& t = THPVariable_Unpack(v.o);
+    if (!t.is_cuda()) return false;
+    out = t.data_ptr();
+    if (dtype) *dtype = t.scalar_type();
+    return true;
+}
+
+bool dtype_code(at::ScalarType t, int& code) {
+    if (t == at::kHalf) code = B200_LORA_F16;
+    else if (t == at::kBFloat16) code = B200_LORA_BF16;
+    else if (t == at::kFloat) code = B200_LORA_F32;
+    else return false;
+    return true;
+}
+
+void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// The adapter table of a pool object, or of a ctypes structure of the same layout.  The ranks are read from
+// the pool's host copy on every call: a pool manager may change a slot's rank between calls.
+bool read_adapters(PyObject* obj, b200_lora_adapters& ad) {
+    if (PyObject_CheckBuffer(obj)) {
+        Py_buffer b;
+        if (PyObject_GetBuffer(obj, &b, PyBUF_SIMPLE) != 0) return false;
+        const bool ok = b.len == (Py_ssize_t)sizeof(ad);
+        if (ok) memcpy(&ad, b.buf, sizeof(ad));
+        PyBuffer_Release(&b);
+        return ok;
+    }
+    memset(&ad, 0, sizeof(ad));
+    int64_t n, l, r, packed;
+    const void *ranks, *scalings, *cum;
+    if (!get_int(obj, s_n_adapters, n) || !get_int(obj, s_n_layers, l) || !get_int(obj, s_r_pool, r) ||
+        !get_int(obj, s_packed, packed) || !get_ptr(obj, s_ranks, true, ranks) ||
+        !get_ptr(obj, s_scalings, true, scalings) || !get_ptr(obj, s_cum_ranks, true, cum))
+        return false;
+    ad.ranks = static_cast<const int32_t*>(ranks);
+    ad.scalings = static_cast<const float*>(scalings);
+    ad.cum_ranks = static_cast<const int64_t*>(cum);
+    ad.n_adapters = (int32_t)n; ad.n_layers = (int32_t)l; ad.r_pool = (int32_t)r; ad.packed = packed ? 1 : 0;
+    ad.scale = 1.0f;
+    Ref rh(PyObject_GetAttr(obj, s_ranks_host)), ch(PyObject_GetAttr(obj, s_cum_host));
+    if (!rh || !ch || !PyObject_CheckBuffer(rh.o) || !PyObject_CheckBuffer(ch.o)) return false;
+    Py_buffer b;
+    if (PyObject_GetBuffer(rh.o, &b, PyBUF_SIMPLE) != 0) return false;
+    bool ok = b.itemsize == 4 && b.len == 4 * n;
+    if (ok) {
+        const int32_t* h = static_cast<const int32_t*>(b.buf);
+        bool pow2 = true;
+        for (int64_t i = 0; i < n; ++i)
+            pow2 &= packed ? (h[i] == 8) | (h[i] == 16) | (h[i] == 32) | (h[i] == 64) : h[i] == (int32_t)r;
+        ad.ranks_pow2 = pow2 && (packed || r == 8 || r == 16 || r == 32 || r == 64);
+    }
+    PyBuffer_Release(&b);
+    if (!ok || PyObject_GetBuffer(ch.o, &b, PyBUF_SIMPLE) != 0) return false;
+    ok = b.itemsize == 8 && b.len >= 8;
+    if (ok) ad.total_rank = static_cast<const int64_t*>(b.buf)[b.len / 8 - 1];
+    PyBuffer_Release(&b);
+    return ok;
+}
+
+struct PlanRef { void* buf; size_t nbytes; int max_tokens; int64_t n_tokens; };
+bool read_plan(PyObject* plan, PlanRef& p) {
+    const void* buf;
+    int64_t nb, cap;
+    if (!get_ptr(plan, s_buf, false, buf) || !get_int(plan, s_nbytes, nb) || !get_int(plan, s_max_tokens, cap) ||
+        !get_int(plan, s_n_tokens, p.n_tokens))
+        return false;
+    p.buf = const_cast<void*>(buf); p.nbytes = (size_t)nb; p.max_tokens = (int)cap;
+    return true;
+}
+
+PyObject* slow() {                 // an attribute or conversion error on the short path is the slow path's to report
+    PyErr_Clear();
+    return PyLong_FromLong(kSlow);
+}
+
+// apply(projs, plan, layer, workspace, flags, adapters | None) -> status
+PyObject* py_apply(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 6) return slow();
+    PyObject* const* items;
+    Py_ssize_t n;
+    if (PyList_CheckExact(args[0])) { items = &PyList_GET_ITEM(args[0], 0); n = PyList_GET_SIZE(args[0]); if (n == 0) return slow(); }
+    else if (PyTuple_CheckExact(args[0])) { n = PyTuple_GET_SIZE(args[0]); if (n == 0) return slow(); items = &PyTuple_GET_ITEM(args[0], 0); }
+    else return slow();
+    if (n > B200_LORA_MAX_PROJ) return slow();
+    PlanRef plan;
+    if (!read_plan(args[1], plan)) return slow();
+    const long layer = PyLong_AsLong(args[2]), flags = PyLong_AsLong(args[4]);
+    if (PyErr_Occurred()) return slow();
+    const void* ws;
+    int64_t ws_bytes;
+    if (!get_ptr(args[3], s_buf, false, ws) || !get_int(args[3], s_nbytes, ws_bytes)) return slow();
+    b200_lora_proj pj[B200_LORA_MAX_PROJ];
+    int io = 0, yd = 0;
+    void* stream = nullptr;
+    PyObject* pool0 = nullptr;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        PyObject* t = items[i];
+        if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 3) return slow();
+        PyObject *ox = PyTuple_GET_ITEM(t, 0), *oy = PyTuple_GET_ITEM(t, 1), *pool = PyTuple_GET_ITEM(t, 2);
+        if (!THPVariable_Check(ox) || !THPVariable_Check(oy)) return slow();
+        const at::Tensor &x = THPVariable_Unpack(ox), &y = THPVariable_Unpack(oy);
+        if (!x.is_cuda() || !y.is_cuda() || x.dim() != 2 || y.dim() != 2) return slow();
+        int64_t h_in, h_out;
+        const void *wa, *wb;
+        at::ScalarType wt;
+        if (!get_int(pool, s_h_in, h_in) || !get_int(pool, s_h_out, h_out) || !get_ptr(pool, s_wa, false, wa, &wt) ||
+            !get_ptr(pool, s_wb, false, wb))
+            return slow();
+        int xi, yi;
+        if (x.size(0) != plan.n_tokens || y.size(0) != plan.n_tokens || x.size(1) != h_in || y.size(1) != h_out ||
+            x.stride(1) != 1 || y.stride(1) != 1 || x.scalar_type() != wt || !dtype_code(x.scalar_type(), xi) ||
+            !dtype_code(y.scalar_type(), yi) || xi == B200_LORA_F32 || (yi != xi && yi != B200_LORA_F32))
+            return slow();
+        if (i == 0) { io = xi; yd = yi; stream = stream_of(x); pool0 = pool; }
+        else if (xi != io || yi != yd) return slow();
+        pj[i] = b200_lora_proj{x.data_ptr(), y.data_ptr(), wa, wb, x.stride(0), y.stride(0), (int32_t)h_in, (int32_t)h_out};
+    }
+    b200_lora_adapters ad;
+    if (!read_adapters(args[5] == Py_None ? pool0 : args[5], ad)) return slow();
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = b200_lora_apply(pj, (int32_t)n, &ad, plan.buf, plan.max_tokens, (int32_t)plan.n_tokens, (int32_t)layer, io, yd, (int32_t)flags,
+                         const_cast<void*>(ws), (size_t)ws_bytes, stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+// plan_build(plan, ids, pool | adapters) -> status; also sets plan.n_tokens
+PyObject* py_plan_build(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    PlanRef plan;
+    b200_lora_adapters ad;
+    if (nargs != 3 || !THPVariable_Check(args[1]) || !read_plan(args[0], plan) || !read_adapters(args[2], ad)) return slow();
+    const at::Tensor& ids = THPVariable_Unpack(args[1]);
+    if (!ids.is_cuda() || !ids.is_contiguous() || (ids.scalar_type() != at::kInt && ids.scalar_type() != at::kLong)) return slow();
+    const int64_t n = ids.numel();
+    Ref num(PyLong_FromLongLong(n));
+    if (!num || PyObject_SetAttr(args[0], s_n_tokens, num.o) != 0) return slow();
+    void* stream = stream_of(ids);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = b200_lora_plan_build(plan.buf, plan.nbytes, plan.max_tokens, ids.data_ptr(), ids.scalar_type() == at::kLong, (int32_t)n, &ad, stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+// plan_segments(plan, seg_starts, seg_adapter, n_tokens, pool | adapters) -> status; also sets plan.n_tokens.
+// seg_starts has more entries than seg_adapter, or as many (then the last segment ends at n_tokens).
+PyObject* py_plan_segments(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    PlanRef plan;
+    b200_lora_adapters ad;
+    if (nargs != 5 || !THPVariable_Check(args[1]) || !THPVariable_Check(args[2]) || !read_plan(args[0], plan) || !read_adapters(args[4], ad))
+        return slow();
+    const at::Tensor &starts = THPVariable_Unpack(args[1]), &owner = THPVariable_Unpack(args[2]);
+    if (!starts.is_cuda() || !owner.is_cuda() || starts.scalar_type() != at::kInt || owner.scalar_type() != at::kInt ||
+        !starts.is_contiguous() || !owner.is_contiguous())
+        return slow();
+    const int64_t n = owner.numel(), t = PyLong_AsLongLong(args[3]);
+    if (PyErr_Occurred() || starts.numel() < n) return slow();
+    if (PyObject_SetAttr(args[0], s_n_tokens, args[3]) != 0) return slow();
+    void* stream = stream_of(starts);
+    const bool ends = starts.numel() > n;
+    const int32_t *sp = static_cast<const int32_t*>(starts.data_ptr()), *op = static_cast<const int32_t*>(owner.data_ptr());
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = (ends ? b200_lora_plan_from_segments : b200_lora_plan_from_requests)(plan.buf, plan.nbytes, plan.max_tokens, sp, op, (int32_t)n,
+                                                                               (int32_t)t, &ad, stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+// ---- the reference's operator call ---------------------------------------------------------------
+// Plan and workspace behind add_lora_bgmv for one (device, stream): the memory belongs to the Python side,
+// which registers it here; what the plan was built from is kept here.  The index tensor is held weakly:
+// its object stays comparable by address, its storage does not stay alive.
+struct OpEntry {
+    void* stream;
+    int device;
+    void *plan, *ws;
+    size_t plan_bytes, ws_bytes;
+    int cap_t, cap_n, cap_h;
+    bool built;
+    c10::weak_intrusive_ptr<c10::TensorImpl> ids;
+    const void* ids_ptr;
+    uint32_t version;
+    int ids_type, t, n, r;
+    float scale;
+    unsigned long long capture;
+    OpEntry() : stream(nullptr), device(-1), plan(nullptr), ws(nullptr), plan_bytes(0), ws_bytes(0), cap_t(0), cap_n(0), cap_h(0), built(false),
+                ids(c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()), ids_ptr(nullptr), version(0), ids_type(0), t(0), n(0), r(0),
+                scale(0.f), capture(0) {}
+};
+std::vector<OpEntry>* g_ops;       // guarded by the GIL; a process has a handful of streams
+
+OpEntry* find_op(void* stream, int device) {
+    for (OpEntry& e : *g_ops)
+        if (e.stream == stream && e.device == device) return &e;
+    return nullptr;
+}
+
+// bgmv_register(stream, device, plan_ptr, plan_bytes, ws_ptr, ws_bytes, cap_t, cap_n, cap_h)
+PyObject* py_bgmv_register(PyObject*, PyObject* args) {
+    unsigned long long stream, plan, ws, plan_bytes, ws_bytes;
+    int device, t, n, h;
+    if (!PyArg_ParseTuple(args, "KiKKKKiii", &stream, &device, &plan, &plan_bytes, &ws, &ws_bytes, &t, &n, &h)) return nullptr;
+    OpEntry* e = find_op(reinterpret_cast<void*>(stream), device);
+    if (!e) { g_ops->emplace_back(); e = &g_ops->back(); }
+    e->stream = reinterpret_cast<void*>(stream); e->device = device;
+    e->plan = reinterpret_cast<void*>(plan); e->plan_bytes = plan_bytes;
+    e->ws = reinterpret_cast<void*>(ws); e->ws_bytes = ws_bytes;
+    e->cap_t = t; e->cap_n = n; e->cap_h = h; e->built = false;
+    Py_RETURN_NONE;
+}
+
+// bgmv_forget(): the plans must be rebuilt on their next use
+PyObject* py_bgmv_forget(PyObject*, PyObject*) {
+    for (OpEntry& e : *g_ops) e.built = false;
+    Py_RETURN_NONE;
+}
+
+struct OpArgs {
+    const at::Tensor *y, *x, *wa, *wb, *ids;
+    int64_t t, n, l, r, h_in, h_out;
+    long layer;
+    double scale;
+    int io;
+};
+// (y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale), checked as the op documents them
+bool read_op(PyObject* const* args, OpArgs& a) {
+    for (int i = 0; i < 5; ++i)
+        if (!THPVariable_Check(args[i])) return false;
+    a.y = &THPVariable_Unpack(args[0]); a.x = &THPVariable_Unpack(args[1]); a.wa = &THPVariable_Unpack(args[2]);
+    a.wb = &THPVariable_Unpack(args[3]); a.ids = &THPVariable_Unpack(args[4]);
+    const at::Tensor &y = *a.y, &x = *a.x, &wa = *a.wa, &wb = *a.wb, &ids = *a.ids;
+    if (!y.is_cuda() || !x.is_cuda() || !wa.is_cuda() || !wb.is_cuda() || !ids.is_cuda()) return false;
+    if (wa.dim() != 4 || wb.dim() != 4 || x.dim() != 2 || y.dim() != 2) return false;
+    a.n = wa.size(0); a.l = wa.size(1); a.r = wa.size(2); a.h_in = wa.size(3); a.h_out = wb.size(2); a.t = x.size(0);
+    if (wb.size(0) != a.n || wb.size(1) != a.l || wb.size(3) != a.r || x.size(1) != a.h_in || y.size(0) != a.t ||
+        y.size(1) != a.h_out || ids.numel() != a.t)
+        return false;
+    if (!y.is_contiguous() || !x.is_contiguous() || !wa.is_contiguous() || !wb.is_contiguous() || !ids.is_contiguous()) return false;
+    const at::ScalarType dt = x.scalar_type();
+    if (y.scalar_type() != dt || wa.scalar_type() != dt || wb.scalar_type() != dt || !dtype_code(dt, a.io) || a.io == B200_LORA_F32) return false;
+    if (ids.scalar_type() != at::kInt && ids.scalar_type() != at::kLong) return false;
+    a.layer = PyLong_AsLong(args[5]);
+    if (PyErr_Occurred()) return false;
+    a.scale = PyFloat_AsDouble(args[6]);
+    return !PyErr_Occurred();
+}
+
+// bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) -> status; kSlow also while this stream's plan
+// and workspace are missing or too small
+PyObject* py_bgmv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    OpArgs a;
+    if (nargs != 7 || !read_op(args, a)) return slow();
+    void* stream = stream_of(*a.x);
+    OpEntry* e = find_op(stream, a.ids->get_device());
+    if (!e || a.t > e->cap_t || a.n > e->cap_n || a.h_in > e->cap_h) return slow();
+    unsigned long long cap = 0;
+    int rc = b200_lora_stream_capture_id(stream, &cap);
+    if (rc) return PyLong_FromLong(rc);
+    const void* ids_ptr = a.ids->data_ptr();
+    const bool versioned = !a.ids->is_inference();                  // inference tensors have no version counter
+    const uint32_t version = versioned ? a.ids->_version() : 0;
+    const int ids_type = (int)a.ids->scalar_type();
+    const float scale = (float)a.scale;
+    c10::TensorImpl* impl = a.ids->unsafeGetTensorImpl();
+    const bool same = e->built && versioned && e->ids._unsafe_get_target() == impl && e->ids_ptr == ids_ptr && e->version == version &&
+                      e->ids_type == ids_type && e->t == a.t && e->n == a.n && e->r == a.r && e->scale == scale && e->capture == cap;
+    b200_lora_adapters ad;
+    memset(&ad, 0, sizeof(ad));
+    ad.n_adapters = (int32_t)a.n; ad.n_layers = (int32_t)a.l; ad.r_pool = (int32_t)a.r; ad.scale = scale;
+    if (!same) {
+        e->built = false;
+        void* plan = e->plan;
+        const size_t pb = e->plan_bytes;
+        const int cap_t = e->cap_t;
+        Py_BEGIN_ALLOW_THREADS
+        rc = b200_lora_plan_build(plan, pb, cap_t, ids_ptr, ids_type == (int)at::kLong, (int32_t)a.t, &ad, stream);
+        Py_END_ALLOW_THREADS
+        if (rc) return PyLong_FromLong(rc);
+        e = find_op(stream, a.ids->get_device());                    // another thread may have registered a stream
+        if (!e || e->plan != plan) return slow();
+        e->built = true;
+        e->ids = c10::weak_intrusive_ptr<c10::TensorImpl>(a.ids->getIntrusivePtr());
+        e->ids_ptr = ids_ptr; e->version = version; e->ids_type = ids_type;
+        e->t = (int)a.t; e->n = (int)a.n; e->r = (int)a.r; e->scale = scale; e->capture = cap;
+    }
+    const b200_lora_proj pj{a.x->data_ptr(), a.y->data_ptr(), a.wa->data_ptr(), a.wb->data_ptr(), a.h_in, a.h_out, (int32_t)a.h_in, (int32_t)a.h_out};
+    void *plan = e->plan, *ws = e->ws;
+    const size_t wb = e->ws_bytes;
+    const int cap_t = e->cap_t;
+    Py_BEGIN_ALLOW_THREADS
+    rc = b200_lora_apply(&pj, 1, &ad, plan, cap_t, (int32_t)a.t, (int32_t)a.layer, a.io, a.io, B200_LORA_NO_TENSOR, ws, wb, stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+// bgmv_static(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) -> status
+PyObject* py_bgmv_static(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    OpArgs a;
+    if (nargs != 7 || !read_op(args, a)) return slow();
+    void* stream = stream_of(*a.x);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = b200_add_lora_bgmv_static(a.y->data_ptr(), a.x->data_ptr(), a.wa->data_ptr(), a.wb->data_ptr(), a.ids->data_ptr(),
+                                   a.ids->scalar_type() == at::kLong, (int32_t)a.t, (int32_t)a.h_in, (int32_t)a.h_out, (int32_t)a.n,
+                                   (int32_t)a.l, (int32_t)a.r, (int32_t)a.layer, (float)a.scale, a.io, stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+PyMethodDef kMethods[] = {
+    {"apply", (PyCFunction)(void*)py_apply, METH_FASTCALL, nullptr},
+    {"plan_build", (PyCFunction)(void*)py_plan_build, METH_FASTCALL, nullptr},
+    {"plan_segments", (PyCFunction)(void*)py_plan_segments, METH_FASTCALL, nullptr},
+    {"bgmv", (PyCFunction)(void*)py_bgmv, METH_FASTCALL, nullptr},
+    {"bgmv_static", (PyCFunction)(void*)py_bgmv_static, METH_FASTCALL, nullptr},
+    {"bgmv_register", py_bgmv_register, METH_VARARGS, nullptr},
+    {"bgmv_forget", py_bgmv_forget, METH_NOARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__b200host(void) {
+    struct { PyObject** slot; const char* name; } names[] = {
+        {&s_wa, "wa"}, {&s_wb, "wb"}, {&s_h_in, "h_in"}, {&s_h_out, "h_out"}, {&s_ranks, "ranks"}, {&s_scalings, "scalings"},
+        {&s_cum_ranks, "cum_ranks"}, {&s_n_adapters, "n_adapters"}, {&s_n_layers, "n_layers"}, {&s_r_pool, "r_pool"},
+        {&s_packed, "packed"}, {&s_ranks_host, "ranks_host"}, {&s_cum_host, "cum_host"}, {&s_buf, "buf"}, {&s_nbytes, "nbytes"},
+        {&s_max_tokens, "max_tokens"}, {&s_n_tokens, "n_tokens"}};
+    for (auto& e : names)
+        if (!(*e.slot = PyUnicode_InternFromString(e.name))) return nullptr;
+    g_ops = new std::vector<OpEntry>();
+    return PyModule_Create(&kModule);
+}

@@ -242,9 +242,8 @@ int b200_lora_plan_build(void* plan, size_t plan_bytes, int32_t max_tokens, cons
     return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
 }
 
-int b200_lora_plan_from_segments(void* plan, size_t plan_bytes, int32_t max_tokens,
-                                 const int32_t* seg_starts, const int32_t* seg_adapter, int32_t n_segs,
-                                 int32_t n_tokens, const b200_lora_adapters* adapters, void* stream) {
+static int plan_from_segments(void* plan, size_t plan_bytes, int32_t max_tokens, const int32_t* seg_starts, const int32_t* seg_adapter,
+                              int32_t n_segs, int32_t n_tokens, int last_end_given, const b200_lora_adapters* adapters, void* stream) {
     if (!plan || !seg_starts || !seg_adapter) return B200_LORA_ERR_NULL;
     int rc = check_adapters(adapters);
     if (rc) return rc;
@@ -252,9 +251,21 @@ int b200_lora_plan_from_segments(void* plan, size_t plan_bytes, int32_t max_toke
     const int cap = max_tokens;
     if (plan_bytes < b200_lora_plan_bytes(cap, adapters->n_adapters)) return B200_LORA_ERR_WORKSPACE;
     if (!aligned16(plan)) return B200_LORA_ERR_ALIGN;
-    cudaError_t e = launch_plan_from_segments(plan, cap, seg_starts, seg_adapter, n_segs, n_tokens,
+    cudaError_t e = launch_plan_from_segments(plan, cap, seg_starts, seg_adapter, n_segs, n_tokens, last_end_given,
                                               plan_adapters(adapters), static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
+}
+
+int b200_lora_plan_from_segments(void* plan, size_t plan_bytes, int32_t max_tokens,
+                                 const int32_t* seg_starts, const int32_t* seg_adapter, int32_t n_segs,
+                                 int32_t n_tokens, const b200_lora_adapters* adapters, void* stream) {
+    return plan_from_segments(plan, plan_bytes, max_tokens, seg_starts, seg_adapter, n_segs, n_tokens, 1, adapters, stream);
+}
+
+int b200_lora_plan_from_requests(void* plan, size_t plan_bytes, int32_t max_tokens,
+                                 const int32_t* start_loc, const int32_t* lora_ids, int32_t n_requests,
+                                 int32_t n_tokens, const b200_lora_adapters* adapters, void* stream) {
+    return plan_from_segments(plan, plan_bytes, max_tokens, start_loc, lora_ids, n_requests, n_tokens, 0, adapters, stream);
 }
 
 int b200_lora_plan_read(const void* plan, int32_t* perm, int32_t* seg_starts, int32_t* seg_adapter,

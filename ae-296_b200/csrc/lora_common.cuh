@@ -292,7 +292,7 @@ struct PlanAdapters {          // what the plan bakes into its unit records
 cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64, int n_tokens,
                               const PlanAdapters& ad, cudaStream_t s);
 cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts, const int* seg_adapter,
-                                      int n_segs, int n_tokens, const PlanAdapters& ad, cudaStream_t s);
+                                      int n_segs, int n_tokens, int last_end_given, const PlanAdapters& ad, cudaStream_t s);
 cudaError_t launch_bgmv(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s);
 cudaError_t launch_bgmv_tma(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s);
 int bgmv_tma_shrink_grid(int n_sm);       // CTAs of the TMA shrink kernel (whoever adds up its split-K slots needs it)

@@ -430,7 +430,7 @@ plan_build_kernel(void* plan, int cap, const void* ids, int T, const PlanAdapter
 
 __global__ void __launch_bounds__(kPlanThreads, 1)
 plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_adapter, int S, int T,
-                     const PlanAdapters ad, int n_scr) {
+                     const PlanAdapters ad, int n_scr, int last_end_given) {
     extern __shared__ int dyn_smem[];                      // working tables, when they fit
     const int N = ad.n_adapters;
     // no early launch of the successor here: the apply kernels read the plan before they wait
@@ -447,7 +447,7 @@ plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_
     __syncthreads();
     // validate: offsets start at 0, end at T, strictly increase; adapters in range
     for (int s = tid; s < S; s += kPlanThreads) {
-        int b = seg_starts[s], e = seg_starts[s + 1], a = seg_adapter[s];
+        int b = seg_starts[s], e = s + 1 < S || last_end_given ? seg_starts[s + 1] : T, a = seg_adapter[s];
         if (b < 0 || e <= b || e > T) smem[40] = 2;
         if (a < 0 || a >= N) smem[40] = 1;
         if (s == 0 && b != 0) smem[40] = 2;
@@ -502,7 +502,7 @@ cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64,
 }
 
 cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts, const int* seg_adapter,
-                                      int n_segs, int n_tokens, const PlanAdapters& ad, cudaStream_t s) {
+                                      int n_segs, int n_tokens, int last_end_given, const PlanAdapters& ad, cudaStream_t s) {
     size_t scr = scratch_ints(n_tokens, n_segs);
     int n_scr = 1;
     if (scr * 4 > 200 * 1024) {
@@ -517,7 +517,7 @@ cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    plan_segments_kernel<<<1, kPlanThreads, n_scr ? scr * 4 : 0, s>>>(plan, cap, seg_starts, seg_adapter, n_segs, n_tokens, ad, n_scr);
+    plan_segments_kernel<<<1, kPlanThreads, n_scr ? scr * 4 : 0, s>>>(plan, cap, seg_starts, seg_adapter, n_segs, n_tokens, ad, n_scr, last_end_given);
     return cudaGetLastError();
 }
 

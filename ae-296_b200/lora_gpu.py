@@ -73,6 +73,7 @@ class Lora_GPU:
         # one plan + workspace per decode batch size in use (built by the first call or by
         # set_indices), one for prefill that grows to the largest batch seen
         self._decode_batch = {}
+        self._decode_stale = set()       # batch sizes whose plan has to be rebuilt (set_indices)
         self._prefill_batch = None
         self._prefill_shape = None
         self._fused = None               # (x identity, layer, prefill) -> the k and v deltas computed with q
@@ -81,7 +82,7 @@ class Lora_GPU:
         """Adapter slot of each decode token for batches of ``len(indices)`` tokens."""
         bsz = indices.numel()
         self.select_inds[bsz - 1] = indices.to(device=f"cuda:{self.device}")
-        self._decode_batch.pop(bsz, None)
+        self._decode_stale.add(bsz)
 
     # ---- the three calls the layer code makes ------------------------------------------
     # The layer code asks for q, k and v of one layer in that order with the same input
@@ -119,10 +120,12 @@ class Lora_GPU:
         bsz = x.shape[0]
         batch = self._decode_batch.get(bsz)
         if batch is None:
-            batch = LoraBatch(bsz, self.batch_size, self.in_size, 3, x.device)
+            batch = self._decode_batch[bsz] = LoraBatch(bsz, self.batch_size, self.in_size, 3, x.device)
+            self._decode_stale.add(bsz)
+        if bsz in self._decode_stale:
             batch.plan.build(self.select_inds[bsz - 1], self._ad_decode)
-            self._decode_batch[bsz] = batch
-        y = torch.zeros(3, bsz, self.output_size, device=x.device, dtype=x.dtype)
+            self._decode_stale.discard(bsz)
+        y = torch.zeros(3, bsz, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
         apply([(x, y[i], self._decode_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace,
               _lib.NO_TENSOR, self._ad_decode)
         return {i: y[i] for i in projs}
@@ -142,7 +145,7 @@ class Lora_GPU:
             slots = torch.arange(bsz, dtype=torch.int32, device=x.device)
             batch.plan.from_segments(starts, slots, rows, self._ad_prefill)
             self._prefill_shape = (bsz, seqlen)
-        y = torch.zeros(3, rows, self.output_size, device=x.device, dtype=x.dtype)
+        y = torch.zeros(3, rows, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
         flags = _lib.MID_ROUND if self.prefill_mid_round else 0
         x2 = x.reshape(rows, hidden)
         apply([(x2, y[i], self._prefill_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace, flags,

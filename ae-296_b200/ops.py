@@ -7,11 +7,15 @@ scalings, packed pools, adapter-sorted segments and fused q/k/v application.
 
 PyTorch is used for device memory and streams only; all arithmetic runs in the CUDA
 library, and there is no fallback path.
+
+The hot calls (``apply``, ``add_lora_bgmv``, ``add_lora_bgmv_static`` and plan building) go through the native
+host path first (``csrc/host.cpp``), which reads the tensors in C++ and costs about a microsecond a call; the
+Python code that follows each of them raises the error of a call that does not qualify, or prepares what is
+missing.
 """
 from __future__ import annotations
 
 import ctypes as C
-import weakref
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -64,33 +68,32 @@ class LoraPlan:
         nbytes = _lib.lib().b200_lora_plan_bytes(self.max_tokens, self.n_adapters)
         if nbytes == 0:
             raise ValueError("bad plan dimensions")
-        self.buf = torch.zeros((nbytes + 15) // 16 * 2, dtype=torch.int64, device=device)
+        self.buf = torch.empty((nbytes + 15) // 16 * 2, dtype=torch.int64, device=device)
+        self.buf[:8].zero_()         # the header: a plan that was never built applies nothing
         self.nbytes = self.buf.numel() * 8
         self._keep = None
         self.n_tokens = 0            # rows of the batch the plan was last built for
 
-    def build(self, ids: torch.Tensor, adapters: Adapters) -> "LoraPlan":
+    def build(self, ids: torch.Tensor, adapters) -> "LoraPlan":
+        """``adapters``: the table as an :class:`_lib.Adapters` structure, or the :class:`AdapterPool` it describes."""
         _require_cuda(ids)
         if ids.dtype not in (torch.int32, torch.int64) or not ids.is_contiguous():
             raise ValueError("ids must be a contiguous int32/int64 tensor")
-        self.n_tokens = int(ids.numel())
-        check(_lib.lib().b200_lora_plan_build(
-            self.buf.data_ptr(), self.nbytes, self.max_tokens, ids.data_ptr(),
-            1 if ids.dtype == torch.int64 else 0, ids.numel(), C.byref(adapters), _stream(ids.device)),
-            "plan_build")
+        check(_lib.host().plan_build(self, ids, adapters), "plan_build")
         return self
 
     def from_segments(self, seg_starts: torch.Tensor, seg_adapter: torch.Tensor, n_tokens: int,
-                      adapters: Adapters) -> "LoraPlan":
+                      adapters) -> "LoraPlan":
+        """``seg_starts`` has one entry per segment and the end of the last one (which may be left out: the
+        last segment then ends at ``n_tokens``).  ``adapters`` as for :meth:`build`."""
         _require_cuda(seg_starts, seg_adapter)
         if seg_starts.dtype != torch.int32 or seg_adapter.dtype != torch.int32:
             raise ValueError("segment tables must be int32")
         self._keep = (seg_starts, seg_adapter)
-        self.n_tokens = int(n_tokens)
-        check(_lib.lib().b200_lora_plan_from_segments(
-            self.buf.data_ptr(), self.nbytes, self.max_tokens, seg_starts.data_ptr(), seg_adapter.data_ptr(),
-            seg_adapter.numel(), int(n_tokens), C.byref(adapters), _stream(seg_starts.device)),
-            "plan_from_segments")
+        rc = _lib.host().plan_segments(self, seg_starts, seg_adapter, int(n_tokens), adapters)
+        if rc > 0:
+            raise ValueError("segment tables are contiguous: one start per segment, and optionally the end of the last")
+        check(rc, "plan_from_segments")
         return self
 
     def read(self) -> Tuple[np.ndarray, np.ndarray, np.ndarray]:
@@ -119,19 +122,27 @@ class LoraWorkspace:
         if nbytes == 0:
             raise ValueError("bad workspace dimensions")
         # 128-byte aligned base: the library's layout aligns v relative to the base address
-        raw = torch.zeros(nbytes + 128, dtype=torch.uint8, device=device)                   # zero-filled once
+        raw = torch.empty(nbytes + 128, dtype=torch.uint8, device=device)
         skew = (-raw.data_ptr()) % 128
         self._raw = raw
         self.buf = raw[skew: skew + nbytes]
         self.nbytes = nbytes
+        # the control words and v start at zero; the split-K partials behind them (30 times the size) are
+        # written before they are read
+        off, size = self._v_region()
+        self.buf[:off + size].zero_()
+
+    def _v_region(self) -> Tuple[int, int]:
+        off, size = C.c_size_t(0), C.c_size_t(0)
+        check(_lib.lib().b200_lora_workspace_v_region(self.max_tokens, self.n_proj, C.byref(off), C.byref(size)),
+              "workspace_v_region")
+        return off.value, size.value
 
     def v_view(self) -> torch.Tensor:
         """The fp32 shrink result ``v [n_proj, max_tokens, 64]`` inside the workspace
         (what tensor-parallel ranks sum between the shrink and the expand half)."""
-        off, size = C.c_size_t(0), C.c_size_t(0)
-        check(_lib.lib().b200_lora_workspace_v_region(self.max_tokens, self.n_proj, C.byref(off), C.byref(size)),
-              "workspace_v_region")
-        return self.buf[off.value: off.value + size.value].view(torch.float32).view(self.n_proj, self.max_tokens, 64)
+        off, size = self._v_region()
+        return self.buf[off: off + size].view(torch.float32).view(self.n_proj, self.max_tokens, 64)
 
 
 def apply(projs: Sequence[Tuple[torch.Tensor, torch.Tensor, AdapterPool]], plan: LoraPlan, layer: int,
@@ -142,6 +153,11 @@ def apply(projs: Sequence[Tuple[torch.Tensor, torch.Tensor, AdapterPool]], plan:
     All pools must share one adapter table (ranks, scalings, layout).  With ``tp_ctx`` (the library's
     peer-exchange context of a tensor-parallel rank) the call is ``b200_lora_apply_tp``: ``x``, ``y`` and the
     pools are this rank's shards and the shrink result is summed over the ranks inside the call."""
+    if tp_ctx is None:
+        rc = _lib.host().apply(projs, plan, layer, workspace, flags, adapters)
+        if rc <= 0:
+            check(rc, "apply")
+            return
     if not 1 <= len(projs) <= _lib.MAX_PROJ:
         raise ValueError("1..4 projections per call")
     arr = (Proj * len(projs))()
@@ -179,56 +195,34 @@ def apply(projs: Sequence[Tuple[torch.Tensor, torch.Tensor, AdapterPool]], plan:
 
 
 # ---- the reference's operator call ---------------------------------------------------------------
-class _OpState:
-    """Plan + workspace behind :func:`add_lora_bgmv` for one (device, stream), and what the plan
-    was built from."""
-
-    def __init__(self):
-        self.batch: Optional[LoraBatch] = None
-        self.dims = (0, 0, 0)            # capacity: tokens, adapters, h_in
-        self.key = None
-        self.ids_ref = None
-
-
-_OP_STATE = {}
+_OP_STATE = {}                       # (device, stream) -> (LoraBatch, capacity: tokens, adapters, h_in)
 
 
 def invalidate_plan_cache() -> None:
     """Forget the plans :func:`add_lora_bgmv` keeps.  Needed only after the contents of an index
     tensor were changed behind torch's back (a custom kernel or a raw pointer write, which do not
     bump the tensor's version counter)."""
-    for st in _OP_STATE.values():
-        st.key, st.ids_ref = None, None
+    _lib.host().bgmv_forget()
 
 
-def _plan_for(ids: torch.Tensor, t: int, n: int, r: int, h_in: int, scale: float, ad: Adapters) -> LoraBatch:
-    """The plan of ``ids``, rebuilt only when it can have changed.
+def _op_state(dev, t: int, n: int, h_in: int) -> None:
+    """Makes the plan and workspace behind :func:`add_lora_bgmv` for the current stream large enough.
 
     The reference's decode loop calls the op 3 x n_layers times per step with the SAME index tensor
     (lightllm/models/lora_gpu.py:138,150,162 with ``select_inds[bsz-1]``).  The plan depends on
-    the ids, N, r and the scale only, so it is kept while the very same tensor object is passed
-    again unmodified (torch's version counter) and rebuilt otherwise.  A plan built outside a
+    the ids, N, r and the scale only, so it is kept while the very same tensor is passed again
+    unmodified (torch's version counter) and rebuilt otherwise.  A plan built outside a
     CUDA-graph capture is never used inside one, nor one capture's plan in another: the capture's
     identifier is part of the key, so every graph contains the build of the plan it applies (its
-    first call) and replays rebuild it from the index tensor's contents of the moment."""
-    dev = ids.device
-    skey = (dev.index, _stream(dev))
-    st = _OP_STATE.get(skey)
-    if st is None:
-        st = _OP_STATE[skey] = _OpState()
-    if st.batch is None or t > st.dims[0] or n > st.dims[1] or h_in > st.dims[2]:
-        st.dims = (max(t, st.dims[0]), max(n, st.dims[1]), max(h_in, st.dims[2]))
-        st.batch = LoraBatch(st.dims[0], st.dims[1], st.dims[2], 1, dev)
-        st.key = None
-    cap = C.c_ulonglong(0)
-    check(_lib.lib().b200_lora_stream_capture_id(_stream(dev), C.byref(cap)), "stream_capture_id")
-    key = (ids.data_ptr(), ids._version, ids.dtype, t, n, r, float(scale), cap.value)
-    same = st.key == key and st.ids_ref is not None and st.ids_ref() is ids
-    if not same:
-        st.batch.plan.build(ids, ad)
-        st.key = key
-        st.ids_ref = weakref.ref(ids)
-    return st.batch
+    first call) and replays rebuild it from the index tensor's contents of the moment.  The key lives in
+    the native host path; the memory is held here."""
+    stream = _stream(dev)
+    _, old = _OP_STATE.get((dev.index, stream), (None, (0, 0, 0)))
+    dims = (max(t, old[0]), max(n, old[1]), max(h_in, old[2]))
+    batch = LoraBatch(*dims, 1, dev)
+    _OP_STATE[dev.index, stream] = (batch, dims)
+    _lib.host().bgmv_register(stream, dev.index, batch.plan.buf.data_ptr(), batch.plan.nbytes,
+                              batch.workspace.buf.data_ptr(), batch.workspace.nbytes, *dims)
 
 
 def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T_all: torch.Tensor,
@@ -242,6 +236,10 @@ def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T
     Two launches (shrink, expand) when the index tensor is the one of the previous call on this
     stream, unmodified; one more (the plan kernel) when it is new.
     """
+    rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
+    if rc <= 0:
+        check(rc, "add_lora_bgmv")
+        return
     _require_cuda(y, x, wa_T_all, wb_T_all, indicies)
     if wa_T_all.dim() != 4 or wb_T_all.dim() != 4:
         raise ValueError("weight pools must be [N, L, r, h_in] and [N, L, h_out, r]")
@@ -259,13 +257,11 @@ def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T
         raise ValueError("fp16 or bf16 tensors of one dtype expected")
     if indicies.dtype not in (torch.int32, torch.int64):
         raise ValueError("indicies must be int32 or int64")
-    ad = _adapters_struct(n, l, r, scale=scale)
-    batch = _plan_for(indicies, t, n, r, h_in, scale, ad)
-    arr = (Proj * 1)(Proj(x.data_ptr(), y.data_ptr(), wa_T_all.data_ptr(), wb_T_all.data_ptr(), h_in, h_out, h_in, h_out))
-    check(_lib.lib().b200_lora_apply(
-        arr, 1, C.byref(ad), batch.plan.buf.data_ptr(), batch.plan.max_tokens, t, int(layer_idx), _DT[x.dtype],
-        _DT[x.dtype], _lib.NO_TENSOR, batch.workspace.buf.data_ptr(), batch.workspace.nbytes, _stream(x.device)),
-        "add_lora_bgmv")
+    _op_state(indicies.device, t, n, h_in)
+    rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
+    if rc > 0:
+        raise ValueError("add_lora_bgmv: unsupported arguments")
+    check(rc, "add_lora_bgmv")
 
 
 def add_lora_bgmv_once(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T_all: torch.Tensor,
@@ -300,6 +296,10 @@ def add_lora_bgmv_static(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tenso
     ``h_in <= 8192`` (larger calls raise).  All calls on a GPU share that one array: issue them
     on one stream, or order the streams, because overlapping calls race.  Make the first call
     on a device outside stream capture (it performs a one-time address lookup)."""
+    rc = _lib.host().bgmv_static(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
+    if rc <= 0:
+        check(rc, "add_lora_bgmv_static")
+        return
     _require_cuda(y, x, wa_T_all, wb_T_all, indicies)
     n, l, r, h_in = wa_T_all.shape
     h_out = wb_T_all.shape[2]
@@ -314,10 +314,7 @@ def add_lora_bgmv_static(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tenso
         raise ValueError("fp16 or bf16 tensors of one dtype expected")
     if indicies.dtype not in (torch.int32, torch.int64):
         raise ValueError("indicies must be int32 or int64")
-    check(_lib.lib().b200_add_lora_bgmv_static(
-        y.data_ptr(), x.data_ptr(), wa_T_all.data_ptr(), wb_T_all.data_ptr(), indicies.data_ptr(),
-        1 if indicies.dtype == torch.int64 else 0, t, h_in, h_out, n, l, r, int(layer_idx), float(scale),
-        _DT[x.dtype], _stream(x.device)), "add_lora_bgmv_static")
+    raise ValueError("add_lora_bgmv_static: unsupported arguments")
 
 
 def add_lora_bgmv_static_status(device=None) -> None:
@@ -339,12 +336,12 @@ class LoraBatch:
     def set_ids(self, ids: torch.Tensor, pool: AdapterPool, tiles: bool = False) -> "LoraBatch":
         """Per-token adapter ids.  ``tiles=True`` also launches the tcgen05 tile kernel for
         tall contiguous runs (mixed prefill + decode batches); decode batches leave it off."""
-        self.plan.build(ids, adapters_of(pool))
+        self.plan.build(ids, pool)
         self.tiles = tiles
         return self
 
     def set_segments(self, seg_starts, seg_adapter, n_tokens, pool: AdapterPool, tiles: bool = True) -> "LoraBatch":
-        self.plan.from_segments(seg_starts, seg_adapter, n_tokens, adapters_of(pool))
+        self.plan.from_segments(seg_starts, seg_adapter, n_tokens, pool)
         self.tiles = tiles
         return self
 

@@ -125,6 +125,12 @@ int b200_lora_plan_from_segments(void* plan, size_t plan_bytes, int32_t max_toke
                                  const int32_t* seg_starts, const int32_t* seg_adapter, int32_t n_segs,
                                  int32_t n_tokens, const b200_lora_adapters* adapters, void* stream);
 
+/* The same from a router's tensors: start_loc [n_requests] holds every request's first row (lightllm's
+ * b_start_loc), the last request ends at n_tokens. */
+int b200_lora_plan_from_requests(void* plan, size_t plan_bytes, int32_t max_tokens,
+                                 const int32_t* start_loc, const int32_t* lora_ids, int32_t n_requests,
+                                 int32_t n_tokens, const b200_lora_adapters* adapters, void* stream);
+
 /* Copies the plan's tables to host arrays (synchronises `stream`): perm [T], seg_starts
  * [T+1], seg_adapter [T]; *n_segs receives S.  Returns B200_LORA_ERR_ID_RANGE if the build
  * saw an id outside [0, N) (such a plan applies nothing). */
