@@ -51,11 +51,12 @@ EncodeTiledFn encode_tiled() {
 // 2-D map over a row-major 16-bit matrix [rows, inner] with row pitch `pitch` elements;
 // cached per (base, shape, box)
 bool tensor_map_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint32_t box_inner,
-                   uint32_t box_rows, CUtensorMapSwizzle swizzle, uint64_t pitch = 0) {
+                   uint32_t box_rows, CUtensorMapSwizzle swizzle, uint64_t pitch = 0,
+                   CUtensorMapL2promotion promote = CU_TENSOR_MAP_L2_PROMOTION_L2_256B) {
     if (pitch == 0) pitch = inner;
     // Encoded maps are kept in a hashed, 4-way set-associative table (4096 entries): an eager loop over
     // many layers presents a few hundred (base pointer, shape) keys per step, and a look-up touches one set.
-    struct Entry { const void* base; uint64_t inner, rows, pitch; uint32_t bi, br; int sw; bool used; CUtensorMap map; };
+    struct Entry { const void* base; uint64_t inner, rows, pitch; uint32_t bi, br; int sw; int promote; bool used; CUtensorMap map; };
     constexpr int kSets = 1024, kWays = 4;
     static Entry cache[kSets][kWays];
     static unsigned char victim[kSets];
@@ -69,7 +70,7 @@ bool tensor_map_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t 
     for (int i = 0; i < kWays; ++i) {
         const Entry& e = set[i];
         if (e.used && e.base == base && e.inner == inner && e.rows == rows && e.pitch == pitch && e.bi == box_inner &&
-            e.br == box_rows && e.sw == (int)swizzle) { *out = e.map; return true; }
+            e.br == box_rows && e.sw == (int)swizzle && e.promote == (int)promote) { *out = e.map; return true; }
     }
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return false;
@@ -79,7 +80,7 @@ bool tensor_map_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t 
     cuuint32_t box[2] = {box_inner, box_rows};
     cuuint32_t estr[2] = {1, 1};
     if (fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promote,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     int way = -1;
@@ -91,6 +92,7 @@ bool tensor_map_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t 
     }
     Entry& e = set[way];
     e.base = base; e.inner = inner; e.rows = rows; e.pitch = pitch; e.bi = box_inner; e.br = box_rows; e.sw = (int)swizzle;
+    e.promote = (int)promote;
     e.used = true; e.map = m;
     *out = m;
     return true;
@@ -412,20 +414,34 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
         }
     }
     bool fast = fast_ranks(adapters);
+    // Dense pools of any other ranks take the TMA kernels' padded form, except where one half runs alone
+    // or the ranks of a group exchange the intermediate (who adds up the split-K slots there works with
+    // the adapters' own ranks).  32 layers of a 93-token decode step, ranks 8 to 64 in R = 64: 3316 us on the
+    // general kernels, 943 us here.
+    const bool padded = !fast && !adapters->packed && !tp && !(flags & (B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND));
+    if (padded) { fast = true; p.flags &= ~B200_LORA_DELTA_THEN_ADD; }   // a flag that these pools do not have
     for (int i = 0; i < n_proj; ++i)
         // units are cut at multiples of 128 columns (the shrink kernel's weight box, the widest
         // per-warp column group of the expand kernel), so the last unit of a row may be partial
         if ((projs[i].h_in % 128) || (projs[i].h_out % 128) || projs[i].h_in > 8192) fast = false;
+    CUtensorMap bmap[kMaxProj][4];
     if (fast) {
+        if (padded) memset(bmap, 0, sizeof(bmap));
         for (int i = 0; i < n_proj && fast; ++i)
             for (int c = 0; c < 4 && fast; ++c) {
                 const uint32_t rc = 8u << c;
-                if (!adapters->packed && rc != (uint32_t)adapters->r_pool) continue;    // dense pools have one rank
-                fast = tensor_map_2d(&p.amap[i][c], projs[i].wa, (uint64_t)projs[i].h_in, pool_rows(adapters), 128, rc,
+                if (padded ? rc >= 2u * adapters->r_pool : !adapters->packed && rc != (uint32_t)adapters->r_pool) continue;    // dense pools have one rank
+                if (padded) {
+                    const uint64_t brows = (uint64_t)adapters->n_adapters * adapters->n_layers * projs[i].h_out;
+                    fast = brows <= 0x7fffffffull &&        // box coordinates are 32-bit
+                           tensor_map_2d(&bmap[i][c], projs[i].wb, (uint64_t)adapters->r_pool, brows, rc, 128,
+                                         CU_TENSOR_MAP_SWIZZLE_NONE, 0, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+                }
+                fast = fast && tensor_map_2d(&p.amap[i][c], projs[i].wa, (uint64_t)projs[i].h_in, pool_rows(adapters), 128, rc,
                                      CU_TENSOR_MAP_SWIZZLE_NONE);
             }
     }
-    auto bgmv = [&](const ApplyParams& q) { return fast ? launch_bgmv_tma(q, io_dtype, n_sm, s) : launch_bgmv(q, io_dtype, n_sm, s); };
+    auto bgmv = [&](const ApplyParams& q) { return fast ? launch_bgmv_tma(q, padded ? bmap : nullptr, io_dtype, n_sm, s) : launch_bgmv(q, io_dtype, n_sm, s); };
     if (e == cudaSuccess && !tp) e = bgmv(p);
     if (e == cudaSuccess && tp) {
         // the TMA shrink kernel leaves its split-K slots and the exchange adds them up; the general one leaves v

@@ -1,7 +1,8 @@
 // Decode BGMV, fast path: TMA copies + mbarrier pipeline + mma.sync (sm_100a).
 //
-// Used when every adapter rank is 8, 16, 32 or 64 and every projection width is a multiple of
-// 256.  One apply is two launches, a shrink kernel (v = x . A^T per work segment) and an expand
+// Used when every projection width is a multiple of 128 and either every adapter rank is 8, 16, 32
+// or 64 (packed pools, dense pools of that one rank) or the pool is dense (any ranks <= R: the PAD
+// instantiations).  One apply is two launches, a shrink kernel (v = x . A^T per work segment) and an expand
 // kernel (y += scale * v . B^T); both are lists of <= 16 KB weight units, ordered projection by
 // projection and work segment by work segment, of which every CTA takes a contiguous range.
 // A CTA is two producer warps plus eight consumer warps around a 4-stage shared-memory ring;
@@ -34,11 +35,24 @@
 // hold the hi and lo 16-bit halves of four tokens' fp32 intermediate, so one MMA is exact for
 // four tokens; results are added into the staged y tile, which each warp writes back itself.
 //
+// PAD: a dense pool [N, L, R, h_in] / [N, L, h_out, R] whose adapters have any rank r <= R.  An
+// adapter is worked on as its rank class 8 / 16 / 32 / 64 (the next one up), with the units, slots
+// and MMA shapes of that class.  Its B rows lie R apart, so the weight tile of an expand unit comes
+// as [128 rows x class] boxes of a 2-D map over the B pool, which pack into the same shared-memory
+// layout as a contiguous block; the map promotes nothing in L2, so a row costs the sectors of its
+// class and not all R columns.  What lies between r and the class is not part of the adapter and may
+// hold anything: those rows of the intermediate are written as zeros when a run is flushed, and those
+// columns of the weight fragments are masked out in registers (a product with zero would let a NaN
+// through).  A 93-token decode step, ranks 8 to 64 in
+// R = 64, 64 applies: 3316 us on the general kernels, 943 us here.
+//
 // Every mbarrier wait is bounded: on expiry the thread records an error word in the workspace
 // and carries on with the same control flow, so the kernel always terminates.
 //
 // Semantics: add_lora_bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) of the
 // reference (lightllm/models/lora_gpu.py:138,150,162), pools as at :33-40.
+#include <string.h>
+
 #include "lora_common.cuh"
 #include "lora_fold.cuh"
 
@@ -113,6 +127,13 @@ __device__ __forceinline__ void tensor_g2s_2d(unsigned dst, const void* tmap, in
                  ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kConsThreads) : "memory"); }
+
+// The rank class whose units, slots and MMA shapes an adapter of rank `r` uses.
+template <bool PAD> __device__ __forceinline__ int rank_class(int r) { return PAD ? pad_rank(r) : r; }
+
+// Maps over the B pools [rows, R], box 128 rows x 8, 16, 32, 64 columns by rank class; padded dense pools only.
+template <bool PAD> struct PadMaps { };
+template <> struct PadMaps<true> { alignas(64) CUtensorMap bmap[kMaxProj][4]; };
 
 template <typename T> struct Mma;
 template <> struct Mma<__half> {
@@ -205,14 +226,15 @@ __device__ __forceinline__ Meta load_meta(const Meta* slot) {
 
 // What the producer derives for one item; every lane computes it from the broadcast record.
 struct Item {
-    int adapter, rank, sub, ntok, start;
+    int adapter, rank, sub, ntok, start;         // rank: its class for padded pools
     long long cum;
     int proj, c0, valid, kc, n_chunks, width_ok;
 };
+template <bool PAD>
 __device__ __forceinline__ Item make_item(const ApplyParams& p, int rec, const Cursor& c, bool expand) {
     Item it;
     it.adapter = __shfl_sync(0xffffffffu, rec, 0);
-    it.rank = __shfl_sync(0xffffffffu, rec, 1);
+    it.rank = rank_class<PAD>(__shfl_sync(0xffffffffu, rec, 1));
     const int w2 = __shfl_sync(0xffffffffu, rec, 2);
     it.sub = c.sub;
     it.ntok = (w2 >> 16) & 0xffff;
@@ -279,9 +301,10 @@ __device__ __forceinline__ void shrink_produce(const ApplyParams& p, const Item&
 
 // An item and its record as the meta slot holds them (for the parts of a unit that are
 // requested after the rest).
+template <bool PAD>
 __device__ __forceinline__ Item item_of_meta(const Meta& m) {
     Item it;
-    it.adapter = m.u.adapter; it.rank = m.u.rank; it.sub = m.u.sub; it.ntok = m.u.ntok; it.start = m.u.start;
+    it.adapter = m.u.adapter; it.rank = rank_class<PAD>(m.u.rank); it.sub = m.u.sub; it.ntok = m.u.ntok; it.start = m.u.start;
     it.cum = ((long long)m.u.cum_hi << 32) | (unsigned)m.u.cum_lo;
     it.proj = m.proj; it.c0 = m.c0; it.valid = m.valid; it.kc = m.kc; it.n_chunks = m.n_chunks; it.width_ok = m.width_ok;
     return it;
@@ -317,9 +340,9 @@ __device__ __forceinline__ void shrink_consume(const Meta& m, const unsigned cha
         }
     }
 }
-template <typename T>
+template <typename T, bool PAD>
 __device__ __forceinline__ void shrink_consume_any(const Meta& m, const unsigned char* stage, float (&acc)[4][4], int tid) {
-    switch (m.u.rank) {
+    switch (rank_class<PAD>(m.u.rank)) {
         case 8:  shrink_consume<T, 8>(m, stage, acc, tid); break;
         case 16: shrink_consume<T, 16>(m, stage, acc, tid); break;
         case 32: shrink_consume<T, 32>(m, stage, acc, tid); break;
@@ -337,13 +360,13 @@ struct Run {
 // so whoever needs the intermediate adds the slots up after this kernel has ended (the expand
 // kernel's producers, or fold_partials_kernel for tensor-parallel callers).  No atomics, no
 // fences; the reduction tile alternates between two buffers, so one barrier per run suffices.
-template <typename T>
+template <bool PAD>
 __device__ __forceinline__ void shrink_flush(const ApplyParams& p, const WorkspaceView& ws, const Run& run,
                                              float (&acc)[4][4], float* red2, int& red_sel, int tid) {
     float* red = red2 + red_sel * (kRedBytes / 4);
     red_sel ^= 1;
     const int lane = tid & 31, warp = tid >> 5;
-    const int r = run.rank, rp = r + 4;
+    const int r = rank_class<PAD>(run.rank), rp = r + 4;
     const int mb_log = r >= 64 ? 2 : r >= 32 ? 1 : 0;
     const int ksplit = kConsWarps >> mb_log;
     const int kslot = warp & (ksplit - 1), mblk = warp >> (3 - mb_log);
@@ -371,11 +394,12 @@ __device__ __forceinline__ void shrink_flush(const ApplyParams& p, const Workspa
         const int tok = idx >> rshift, i = idx & (r - 1);
         float s = 0.f;
         for (int w = 0; w < ksplit; ++w) s += red[(w * 8 + tok) * rp + i];
+        if (PAD && i >= run.rank) s = 0.f;                  // rows of the class that are not the adapter's
         dst[tok * kMaxRank + i] = s;
     }
 }
 
-template <typename T>
+template <typename T, bool PAD>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_shrink_tma_kernel(const __grid_constant__ ApplyParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     float* red2 = reinterpret_cast<float*>(smem + kStages * kShrinkStage);      // two reduction tiles
@@ -426,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_shrink_tma_kernel(c
             for (int k = pw; k < upto; k += kProdWarps) {
                 const Meta& mk = meta[k % kMetaSlots];
                 if (mk.valid)
-                    shrink_produce<T>(p, item_of_meta(mk), record_of_meta(mk, lane), smem_u32(smem + (k % kStages) * kShrinkStage),
+                    shrink_produce<T>(p, item_of_meta<PAD>(mk), record_of_meta(mk, lane), smem_u32(smem + (k % kStages) * kShrinkStage),
                                       smem_u32(&bars[k % kStages]), lane, 2);
             }
         };
@@ -434,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_shrink_tma_kernel(c
             if (!waited && n >= kStages) late_parts(n);
             const int s = n % kStages;
             const unsigned ph = (n / kStages) & 1;
-            const Item it = make_item(p, rec, cur, false);
+            const Item it = make_item<PAD>(p, rec, cur, false);
             // There are twice as many meta slots as stages, so unit n's slot is free once unit
             // n - kStages has been handed over: fill it before waiting for the stage itself, and
             // nothing but the copies stands between that wait and the stage being in flight again.
@@ -466,17 +490,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_shrink_tma_kernel(c
         const Meta m = load_meta(&meta[n % kMetaSlots]);
         if (m.valid) {
             if (m.proj != run.proj || m.u.wseg != run.wseg) {
-                if (run.count > 0) shrink_flush<T>(p, ws, run, acc, red2, red_sel, tid);
+                if (run.count > 0) shrink_flush<PAD>(p, ws, run, acc, red2, red_sel, tid);
                 run.proj = m.proj; run.wseg = m.u.wseg; run.start = m.u.start; run.ntok = m.u.ntok;
                 run.rank = m.u.rank; run.first_kc = m.kc; run.count = 0; run.n_chunks = m.n_chunks;
             }
-            shrink_consume_any<T>(m, smem + s * kShrinkStage, acc, tid);
+            shrink_consume_any<T, PAD>(m, smem + s * kShrinkStage, acc, tid);
             ++run.count;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars[kStages + s]));      // this warp is done with the stage
     }
-    if (run.count > 0) shrink_flush<T>(p, ws, run, acc, red2, red_sel, tid);
+    if (run.count > 0) shrink_flush<PAD>(p, ws, run, acc, red2, red_sel, tid);
 }
 
 // =============================================================================================
@@ -496,8 +520,8 @@ struct FoldCtx {
 // fragments for the units that follow - and comes either from the workspace (a tensor-parallel
 // caller has summed it over the ranks) or from the shrink kernel's split-K slots, which the
 // producer warp adds up in ascending k order straight into the stage.
-template <typename T>
-__device__ __forceinline__ void expand_produce(const ApplyParams& p, const WorkspaceView& ws, const Item& m, int rec,
+template <typename T, bool PAD>
+__device__ __forceinline__ void expand_produce(const ApplyParams& p, const PadMaps<PAD>& pm, const WorkspaceView& ws, const Item& m, int rec,
                                                unsigned char* stage_ptr, unsigned bar, int lane, int parts, bool need_v,
                                                const FoldCtx& fc, int u0) {
     const unsigned stage = smem_u32(stage_ptr);
@@ -512,11 +536,17 @@ __device__ __forceinline__ void expand_produce(const ApplyParams& p, const Works
         if (lane == 0) mbar_expect_tx(bar, w_bytes + m.ntok * (y_bytes + v_bytes));
         __syncwarp();
     }
+    if constexpr (PAD) {                                   // the weight tile row by row of its class, 128 rows a box
+        const int cls = r <= 8 ? 0 : r <= 16 ? 1 : r <= 32 ? 2 : 3;
+        if ((parts & 1) && lane < m.width_ok / 128)
+            tensor_g2s_2d(stage + lane * (128 * r * 2), &pm.bmap[m.proj][cls], 0,
+                          (int)((m.adapter * (long long)p.n_layers + p.layer) * pj.h_out + m.c0 + lane * 128), bar);
+    }
     // one instruction: lane 0 the weight tile, lanes 8..15 the y rows, lanes 16..23 the v rows
     const int tok = __shfl_sync(0xffffffffu, rec, 8 + (lane & 7));
     unsigned dst = 0, bytes = 0;
     const void* src = pj.wb;
-    if (lane == 0) {
+    if (!PAD && lane == 0) {
         dst = stage;
         src = reinterpret_cast<const T*>(pj.wb) + (item_row0(p, m) * (long long)pj.h_out + (long long)m.c0 * r);
         bytes = (parts & 1) ? w_bytes : 0u;
@@ -581,7 +611,7 @@ __device__ __forceinline__ unsigned hl_pack(float v0, float v1, bool lo) {
 // A warp first moves everything it needs of the stage into registers (intermediate fragments,
 // weight fragments, the staged y values), hands the stage back (`empty_bar`) and only then
 // computes: the time a stage stays out of flight does not include the arithmetic.
-template <typename T, int R>
+template <typename T, int R, bool PAD>
 __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta& m, const int* tok_rows, unsigned char* stage,
                                                int tid, unsigned (&bf)[2][4][2], bool reuse, unsigned empty_bar) {
     constexpr int KS = R == 64 ? 4 : R == 32 ? 2 : 1;
@@ -662,6 +692,21 @@ __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta&
             a[nb][0][0] = *reinterpret_cast<const unsigned*>(w0 + t * 4);
             a[nb][0][1] = *reinterpret_cast<const unsigned*>(w1 + t * 4);
             a[nb][0][2] = a[nb][0][3] = 0u;
+        }
+    }
+    if constexpr (PAD) {                                   // the columns from the adapter's rank on are not its weights
+        if (m.u.rank < R) {
+            // pair j of the thread's k-step k starts at this rank index (the wide loads above)
+            constexpr int per_t = R == 64 ? 16 : R == 32 ? 8 : R == 16 ? 4 : 2;
+#pragma unroll
+            for (int k = 0; k < KS; ++k)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int k0 = t * per_t + k * 4 + j * 2;
+                    const unsigned mask = k0 + 1 < m.u.rank ? 0xffffffffu : k0 < m.u.rank ? 0xffffu : 0u;
+#pragma unroll
+                    for (int nb = 0; nb < NBW; ++nb) { a[nb][k][2 * j] &= mask; a[nb][k][2 * j + 1] &= mask; }
+                }
         }
     }
     // Token t (+4): hi + lo products for columns g and g + 8.  Lanes g and g ^ 1 swap one value
@@ -746,8 +791,9 @@ __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta&
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(const __grid_constant__ ApplyParams p) {
+template <typename T, bool PAD>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+bgmv_expand_tma_kernel(const __grid_constant__ ApplyParams p, const __grid_constant__ PadMaps<PAD> pm) {
     extern __shared__ __align__(1024) unsigned char smem[];
     Meta* meta = reinterpret_cast<Meta*>(smem + kStages * kExpandStage);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(meta + kMetaSlots);
@@ -798,7 +844,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(c
             for (int k = pw; k < upto; k += kProdWarps) {
                 const Meta& mk = meta[k % kMetaSlots];
                 if (mk.valid)
-                    expand_produce<T>(p, ws, item_of_meta(mk), record_of_meta(mk, lane), smem + (k % kStages) * kExpandStage,
+                    expand_produce<T, PAD>(p, pm, ws, item_of_meta<PAD>(mk), record_of_meta(mk, lane), smem + (k % kStages) * kExpandStage,
                                       smem_u32(&bars[k % kStages]), lane, 2, mk.pad[0] != 0, fc, mk.pad[1]);
             }
         };
@@ -806,7 +852,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(c
             if (!waited && n >= kStages) late_parts(n);
             const int s = n % kStages;
             const unsigned ph = (n / kStages) & 1;
-            const Item it = make_item(p, rec, cur, true);
+            const Item it = make_item<PAD>(p, rec, cur, true);
             // the CTA's first unit of a (projection, work segment) brings the intermediate along
             const bool need_v = n == 0 || (cur.sp == 0 && cur.sub == 0);
             // ... except the CTA's very first unit, whose intermediate the (still idle) consumer
@@ -819,7 +865,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(c
             if (n == 0) asm volatile("bar.arrive 2, %0;" ::"n"(kConsThreads + 32) : "memory");   // meta slot 0 is published
             mbar_wait(smem_u32(&bars[kStages + s]), ph ^ 1, err, 3);
             const unsigned full = smem_u32(&bars[s]);
-            if (it.valid) expand_produce<T>(p, ws, it, rec, smem + s * kExpandStage, full, lane, waited ? 7 : 1 | 4, need_v && !by_consumers, fc, cur.unit);
+            if (it.valid) expand_produce<T, PAD>(p, pm, ws, it, rec, smem + s * kExpandStage, full, lane, waited ? 7 : 1 | 4, need_v && !by_consumers, fc, cur.unit);
             else if (lane == 0) mbar_arrive(full);
             if (n + kProdWarps < n_local) cursor_advance(p, n_units, true, pv.unit_tab, lane, kProdWarps, cur, rec);
         }
@@ -832,7 +878,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(c
     if (!(p.flags & B200_LORA_ONLY_EXPAND)) {
         const Meta m0 = load_meta(&meta[0]);
         if (m0.valid) {
-            const int r = m0.u.rank;
+            const int r = rank_class<PAD>(m0.u.rank);
             const int per_a = (n_units * p.total_super_in + (int)gridDim.x - 1) / (int)gridDim.x;
             const int seg_first = shrink_seg_first(p, n_units, m0.proj, m0.pad[1]);
             const int n_chunks = shrink_chunks(p, m0.proj, r);
@@ -862,11 +908,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bgmv_expand_tma_kernel(c
             const bool reuse = key == bf_key;
             bf_key = key;
             const unsigned empty_bar = smem_u32(&bars[kStages + s]);      // one arrival per consumer warp, made inside
-            switch (m.u.rank) {
-                case 8:  expand_consume<T, 8>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
-                case 16: expand_consume<T, 16>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
-                case 32: expand_consume<T, 32>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
-                default: expand_consume<T, 64>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
+            switch (rank_class<PAD>(m.u.rank)) {
+                case 8:  expand_consume<T, 8, PAD>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
+                case 16: expand_consume<T, 16, PAD>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
+                case 32: expand_consume<T, 32, PAD>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
+                default: expand_consume<T, 64, PAD>(p, m, meta[n % kMetaSlots].u.tok, stage, tid, bf, reuse, empty_bar); break;
             }
         } else {
             __syncwarp();
@@ -929,27 +975,29 @@ static_assert(kCtasPerSm * (kShrinkSmem + 1024) <= 233472 && kCtasPerSm * (kExpa
 // shrink kernel, then expand kernel (whose producers add up the split-K slots), each launched so
 // that its prologue and first weight copies overlap its predecessor's tail; callers that want
 // only one half get that half, and after a lone shrink half the intermediate is written out.
-template <typename T>
-cudaError_t launch_pair(const ApplyParams& p, int n_sm, cudaStream_t s) {
+template <typename T, bool PAD>
+cudaError_t launch_pair(const ApplyParams& p, const PadMaps<PAD>& pm, int n_sm, cudaStream_t s) {
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(bgmv_shrink_tma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShrinkSmem);
+        cudaError_t e = cudaFuncSetAttribute(bgmv_shrink_tma_kernel<T, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kShrinkSmem);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(bgmv_expand_tma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpandSmem);
+        e = cudaFuncSetAttribute(bgmv_expand_tma_kernel<T, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpandSmem);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     const int grid = n_sm * kCtasPerSm;
     cudaError_t e = cudaSuccess;
     if (!(p.flags & B200_LORA_ONLY_EXPAND)) {
-        e = launch_pdl(bgmv_shrink_tma_kernel<T>, grid, kThreads, kShrinkSmem, s, p);
-        if (e == cudaSuccess && (p.flags & B200_LORA_ONLY_SHRINK) && !(p.flags & B200_LORA_KEEP_PARTIALS))
-            e = launch_pdl(fold_partials_kernel<T>, dim3(n_sm, p.n_proj), 128, 0, s, p, grid);
+        e = launch_pdl(bgmv_shrink_tma_kernel<T, PAD>, grid, kThreads, kShrinkSmem, s, p);
+        if constexpr (!PAD) {
+            if (e == cudaSuccess && (p.flags & B200_LORA_ONLY_SHRINK) && !(p.flags & B200_LORA_KEEP_PARTIALS))
+                e = launch_pdl(fold_partials_kernel<T>, dim3(n_sm, p.n_proj), 128, 0, s, p, grid);
+        }
     }
     if (e == cudaSuccess && !(p.flags & B200_LORA_ONLY_SHRINK))
-        e = launch_pdl(bgmv_expand_tma_kernel<T>, grid, kThreads, kExpandSmem, s, p);
+        e = launch_pdl(bgmv_expand_tma_kernel<T, PAD>, grid, kThreads, kExpandSmem, s, p, pm);
     return e;
 }
 
@@ -957,9 +1005,15 @@ cudaError_t launch_pair(const ApplyParams& p, int n_sm, cudaStream_t s) {
 
 int bgmv_tma_shrink_grid(int n_sm) { return n_sm * kCtasPerSm; }
 
-cudaError_t launch_bgmv_tma(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s) {
-    if (io_dtype == B200_LORA_F16) return launch_pair<__half>(p, n_sm, s);
-    return launch_pair<__nv_bfloat16>(p, n_sm, s);
+cudaError_t launch_bgmv_tma(const ApplyParams& p, const CUtensorMap (*bmap)[4], int io_dtype, int n_sm, cudaStream_t s) {
+    if (!bmap) {
+        if (io_dtype == B200_LORA_F16) return launch_pair<__half, false>(p, PadMaps<false>(), n_sm, s);
+        return launch_pair<__nv_bfloat16, false>(p, PadMaps<false>(), n_sm, s);
+    }
+    PadMaps<true> pm;
+    memcpy(pm.bmap, bmap, sizeof(pm.bmap));
+    if (io_dtype == B200_LORA_F16) return launch_pair<__half, true>(p, pm, n_sm, s);
+    return launch_pair<__nv_bfloat16, true>(p, pm, n_sm, s);
 }
 
 }  // namespace b200lora

@@ -294,7 +294,8 @@ cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64,
 cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts, const int* seg_adapter,
                                       int n_segs, int n_tokens, int last_end_given, const PlanAdapters& ad, cudaStream_t s);
 cudaError_t launch_bgmv(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s);
-cudaError_t launch_bgmv_tma(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s);
+// `bmap` (padded dense pools): maps over the B pools, box 128 rows x rank class; NULL: contiguous B blocks
+cudaError_t launch_bgmv_tma(const ApplyParams& p, const CUtensorMap (*bmap)[4], int io_dtype, int n_sm, cudaStream_t s);
 int bgmv_tma_shrink_grid(int n_sm);       // CTAs of the TMA shrink kernel (whoever adds up its split-K slots needs it)
 cudaError_t launch_tp_exchange(const b200_lora_tp* tp, void* workspace, int n_proj, int cap, int n_tokens, int skip_push,
                                int n_sm, cudaStream_t s);

@@ -47,6 +47,23 @@ def test_dense_pool_ranks_not_multiple_of_8_and_garbage_padding():
     assert rel_err(y32.double().cpu().numpy(), c.oracle_delta(0)) <= TOL
 
 
+@pytest.mark.parametrize("r_max,ranks", [(8, [1, 7, 8]), (16, [9, 15, 16, 2]), (24, [24, 17, 8, 3]), (40, [40, 33, 16, 5]),
+                                         (64, [63, 31, 12, 64])])
+@pytest.mark.parametrize("T,h_in,h_out,dtype", [(1, 128, 640, "fp16"), (9, 640, 128, "bf16"), (70, 2176, 2432, "fp16")])
+def test_padded_dense_pools_of_any_rank(r_max, ranks, T, h_in, h_out, dtype):
+    """Dense pools R that hold ranks below R: every rank class and its edges, R itself below its class, partial
+    units and partial super-chunks, one to full work segments; what lies beyond an adapter's rank is NaN."""
+    c = Case(T, len(ranks), h_in, h_out, np.array(ranks, np.int32), dtype, dense=True, seed=r_max + T)
+    assert c.pool.r_pool == r_max
+    for a, r in enumerate(ranks):
+        c.pool.wa[a, :, r:, :] = float("nan")
+        c.pool.wb[a, :, :, r:] = float("nan")
+    for layer in (0, c.n_layers - 1):
+        y32 = c.run(layer, y_dtype=torch.float32)
+        assert rel_err(y32.double().cpu().numpy(), c.oracle_delta(layer)) <= TOL
+        assert torch.equal(c.run(layer), y32.to(c.tdt))
+
+
 def test_accumulates_into_y_with_strides_and_canaries():
     c = Case(37, 9, 640, 384, [16, 32], "bf16", seed=11)
     g = torch.Generator().manual_seed(5)
