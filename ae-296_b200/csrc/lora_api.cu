@@ -160,6 +160,30 @@ bool fast_ranks(const b200_lora_adapters* ad) {
     return ad->ranks_pow2 != 0 && (ad->packed || pow2);
 }
 
+// Does the one-launch cluster kernel take this apply?  Yes while all its clusters (at most a segment per
+// token, times the projections) run at once: each is a chain that is much longer than its bytes take, and a
+// second round of clusters would pay the chain again, while the two streaming kernels only get longer.
+// Microseconds per apply, two kernels / cluster kernel, distinct adapters, graph replay (items = tokens x projections):
+//   h 4096, r 16 (3 CTAs an SM):  1 item 5.5 / 3.6   24 items 7.6 / 4.7   48 items 8.8 / 7.4   64 items 9.7 / 10.5
+//   h 4096, r 64 (1 CTA an SM):   1 item 6.8 / 5.0   12 items 9.5 / 6.9   16 items 10.4 / 11.9
+//   h 2048, r 64 (2 CTAs an SM):  1 item 6.1 / 4.7   24 items 9.1 / 6.8   32 items 9.9 / 8.3   36 items 10.2 / 11.7
+// and bgmv_cluster_limit() is 48 to 54, 14 to 18 and 28 to 36 there.
+bool cluster_route(const ApplyParams& p, const b200_lora_adapters* ad, int io_dtype) {
+    if ((long long)p.n_tokens * p.n_proj > 1024) return false;       // far beyond any limit
+    const int other = B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND | B200_LORA_DELTA_THEN_ADD;
+    if (!(p.flags & B200_LORA_NO_TENSOR) || (p.flags & other) || !fast_ranks(ad) || !bgmv_cluster_fits(p)) return false;
+    // a cluster writes its y rows while others still read x: not when the two share memory
+    for (int i = 0; i < p.n_proj; ++i)
+        for (int j = 0; j < p.n_proj; ++j) {
+            const ProjArgs &a = p.proj[i], &b = p.proj[j];
+            const uintptr_t x0 = reinterpret_cast<uintptr_t>(a.x), y0 = reinterpret_cast<uintptr_t>(b.y);
+            const uintptr_t x1 = x0 + 2 * ((uintptr_t)(p.n_tokens - 1) * a.ldx + a.h_in);
+            const uintptr_t y1 = y0 + (p.y_f32 ? 4 : 2) * ((uintptr_t)(p.n_tokens - 1) * b.ldy + b.h_out);
+            if (x0 < y1 && y0 < x1) return false;
+        }
+    return p.n_tokens * p.n_proj <= bgmv_cluster_limit(p, io_dtype);
+}
+
 // the workspace's sticky error word as a status code
 int status_of_error_word(unsigned word) {
     if (word == 0u) return B200_LORA_OK;
@@ -370,7 +394,12 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
     const int n_sm = sm_count();
     cudaError_t e = cudaSuccess;
     SideStream* side = nullptr;
-    if (!sgmv_tiles_supported(p)) p.flags |= B200_LORA_NO_TENSOR;
+    // a batch shorter than the shortest tall run has none: no tile launches, no side stream
+    if (!sgmv_tiles_supported(p) || n_tokens < kTallMin) p.flags |= B200_LORA_NO_TENSOR;
+    if (!tp && cluster_route(p, adapters, io_dtype)) {
+        e = launch_bgmv_cluster(p, io_dtype, s);
+        return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
+    }
     if (!(p.flags & B200_LORA_NO_TENSOR)) {
         SgmvParams sp;
         memset(&sp, 0, sizeof(sp));

@@ -66,6 +66,7 @@ struct PlanView {
     int* ws_rank;       // [cap]
     int* ws_unit0;      // [cap]       first unit record of the work segment
     int* unit_tab;      // [16 * cap][16]  one record per weight unit (see UnitRec)
+    int* seg_tab;       // [cap][16]   one unit record per work segment, in the order of the unit list
     int* tile_tab;      // [cap]       two words per tile of a tall run: first sorted position, (seg << 8) | (rows - 1)
     int* hist;          // [n_adapters + 1]
 };
@@ -73,7 +74,7 @@ struct PlanView {
 __host__ __device__ inline size_t plan_words(int cap, int n_adapters) {
     // header + perm + seg_start + 3 seg arrays + units + tiles + hist, each padded to 4 words
     auto pad4 = [](size_t w) { return (w + 3) & ~size_t(3); };
-    return 16 + pad4(cap) + 2 * pad4(cap + 1) + 6 * pad4(cap) + 16 * kMaxSub * (size_t)cap + pad4(cap) +
+    return 16 + pad4(cap) + 2 * pad4(cap + 1) + 6 * pad4(cap) + 16 * kMaxSub * (size_t)cap + 16 * (size_t)cap + pad4(cap) +
            pad4((size_t)n_adapters + 1);
 }
 
@@ -92,6 +93,7 @@ __host__ __device__ inline PlanView plan_view(void* base, int cap, int n_adapter
     v.ws_rank = w;                                 w += pad4(cap);
     v.ws_unit0 = w;                                w += pad4(cap);
     v.unit_tab = w;                                w += 16 * kMaxSub * (size_t)cap;
+    v.seg_tab = w;                                 w += 16 * (size_t)cap;
     v.tile_tab = w;                                w += pad4(cap);
     v.hist = w;
     (void)n_adapters;
@@ -297,6 +299,10 @@ cudaError_t launch_bgmv(const ApplyParams& p, int io_dtype, int n_sm, cudaStream
 // `bmap` (padded dense pools): maps over the B pools, box 128 rows x rank class; NULL: contiguous B blocks
 cudaError_t launch_bgmv_tma(const ApplyParams& p, const CUtensorMap (*bmap)[4], int io_dtype, int n_sm, cudaStream_t s);
 int bgmv_tma_shrink_grid(int n_sm);       // CTAs of the TMA shrink kernel (whoever adds up its split-K slots needs it)
+// one launch per apply for a few tokens (a thread-block cluster per work segment and projection)
+bool bgmv_cluster_fits(const ApplyParams& p);     // widths and shared memory
+int bgmv_cluster_limit(const ApplyParams& p, int io_dtype);      // clusters of this size that run at once
+cudaError_t launch_bgmv_cluster(const ApplyParams& p, int io_dtype, cudaStream_t s);
 cudaError_t launch_tp_exchange(const b200_lora_tp* tp, void* workspace, int n_proj, int cap, int n_tokens, int skip_push,
                                int n_sm, cudaStream_t s);
 // one exchange of a tensor-parallel apply: the rows of the plan's tiles (`tall`) or of its BGMV work segments

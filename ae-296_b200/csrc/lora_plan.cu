@@ -354,7 +354,8 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     }
     __syncthreads();
     // unit records: one work segment per thread, n_sub records of four 16-byte stores each
-    for (int w = tid; w < tot_ws; w += kPlanThreads) {
+    for (int i = tid; i < tot_ws; i += kPlanThreads) {
+        const int w = (int)(((long long)i * stride) % tot_ws);
         const int cb = sc.ws_start[w], ce = sc.ws_start[w + 1];
         const int a = sc.ws_adapter[w], r = sc.ws_rank[w] & 0xffff;
         const int nsub = n_sub(pad_rank(r));
@@ -363,7 +364,10 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
         rec.adapter = a; rec.rank = r; rec.sub = 0; rec.ntok = (short)(ce - cb); rec.wseg = w; rec.start = cb;
         rec.scale = ad.scalings ? ad.scalings[a] : ad.scale;
         rec.cum_lo = (int)(cum & 0xffffffffll); rec.cum_hi = (int)(cum >> 32);
-        for (int i = 0; i < 8; ++i) rec.tok[i] = perm[cb + min(i, ce - cb - 1)];
+        for (int k = 0; k < 8; ++k) rec.tok[k] = perm[cb + min(k, ce - cb - 1)];
+        uint4* seg = reinterpret_cast<uint4*>(reinterpret_cast<UnitRec*>(pv.seg_tab) + i);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) seg[q] = reinterpret_cast<const uint4*>(&rec)[q];
         uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<UnitRec*>(pv.unit_tab) + sc.ws_unit0[w]);
         for (int j = 0; j < nsub; ++j) {
             rec.sub = (short)j;

@@ -47,6 +47,41 @@ def test_dense_pool_ranks_not_multiple_of_8_and_garbage_padding():
     assert rel_err(y32.double().cpu().numpy(), c.oracle_delta(0)) <= TOL
 
 
+@pytest.mark.parametrize("h_in,h_out", [(128, 128), (640, 1152), (1152, 640), (2048, 8192), (8192, 1024)])
+@pytest.mark.parametrize("T,N,ranks,dtype", [(1, 1, [64], "bf16"), (8, 1, [8], "fp16"), (5, 2, [32, 16], "bf16"), (10, 4, [8, 64, 16, 32], "fp16")])
+def test_few_tokens_in_one_launch(T, N, ranks, dtype, h_in, h_out):
+    """The cluster kernel: every rank, one to eight tokens a segment, slices of h_in and h_out that are empty or
+    uneven over the eight CTAs, two projections; and the streaming kernels on the same rows (a batch too large
+    for the cluster route) within fp32 rounding."""
+    ids = np.arange(T) % N
+    c = Case(T, N, h_in, h_out, np.array(ranks, np.int32), dtype, seed=T + h_in, ids=ids)
+    y32 = c.run(1, y_dtype=torch.float32)
+    assert rel_err(y32.double().cpu().numpy(), c.oracle_delta(1)) <= TOL
+    assert torch.equal(c.run(1), y32.to(c.tdt))
+    assert torch.equal(c.run(1, y_dtype=torch.float32), y32)
+    if dtype == "fp16":                   # (a bf16 tie that falls the other way is larger than the bound)
+        assert rel_err(c.run(1, y_dtype=torch.float32, flags=L.MID_ROUND).double().cpu().numpy(), c.oracle_delta(1, mid_round=dtype)) <= TOL
+    ys = [torch.ones(T, h_out, dtype=c.tdt, device="cuda") for _ in range(2)]
+    L.LoraBatch(T, N, h_in, 2).set_ids(c.ids_dev, c.pool).apply([(c.x, y, c.pool) for y in ys], 1)
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], (y32 + 1).to(c.tdt))
+    reps = 200 // T + 1
+    big = torch.zeros(reps * T, h_out, dtype=torch.float32, device="cuda")
+    L.LoraBatch(reps * T, N, h_in, 1).set_ids(c.ids_dev.repeat(reps), c.pool).apply([(c.x.repeat(reps, 1), big, c.pool)], 1)
+    assert rel_err(big[:T].double().cpu().numpy(), y32.double().cpu().numpy()) <= 1e-5
+
+
+def test_few_tokens_with_y_in_the_memory_of_x():
+    """y += delta(x) with y the same rows as x: every projection still sees the old x."""
+    c = Case(6, 3, 512, 512, [16], "fp16", seed=77)
+    want = O.round_to(c.x_cpu.double().numpy() + c.oracle_delta(0), "fp16")
+    y2 = torch.zeros(6, 512, dtype=torch.float16, device="cuda")
+    c_x = c.x.clone()
+    L.LoraBatch(6, 3, 512, 2).set_ids(c.ids_dev, c.pool).apply([(c_x, c_x, c.pool), (c_x, y2, c.pool)], 0)
+    assert np.abs(c_x.double().cpu().numpy() - want).max() <= np.abs(want).max() * 2 ** -10
+    delta = c.oracle_delta(0)
+    assert np.abs(y2.double().cpu().numpy() - delta).max() <= np.abs(delta).max() * 2 ** -10
+
+
 @pytest.mark.parametrize("r_max,ranks", [(8, [1, 7, 8]), (16, [9, 15, 16, 2]), (24, [24, 17, 8, 3]), (40, [40, 33, 16, 5]),
                                          (64, [63, 31, 12, 64])])
 @pytest.mark.parametrize("T,h_in,h_out,dtype", [(1, 128, 640, "fp16"), (9, 640, 128, "bf16"), (70, 2176, 2432, "fp16")])
