@@ -52,7 +52,7 @@ def test_dense_pool_ranks_not_multiple_of_8_and_garbage_padding():
 def test_few_tokens_in_one_launch(T, N, ranks, dtype, h_in, h_out):
     """The cluster kernel: every rank, one to eight tokens a segment, slices of h_in and h_out that are empty or
     uneven over the eight CTAs, two projections; and the streaming kernels on the same rows (a batch too large
-    for the cluster route) within fp32 rounding."""
+    for the cluster route) to the precision both keep v in."""
     ids = np.arange(T) % N
     c = Case(T, N, h_in, h_out, np.array(ranks, np.int32), dtype, seed=T + h_in, ids=ids)
     y32 = c.run(1, y_dtype=torch.float32)
@@ -67,7 +67,9 @@ def test_few_tokens_in_one_launch(T, N, ranks, dtype, h_in, h_out):
     reps = 200 // T + 1
     big = torch.zeros(reps * T, h_out, dtype=torch.float32, device="cuda")
     L.LoraBatch(reps * T, N, h_in, 1).set_ids(c.ids_dev.repeat(reps), c.pool).apply([(c.x.repeat(reps, 1), big, c.pool)], 1)
-    assert rel_err(big[:T].double().cpu().numpy(), y32.double().cpu().numpy()) <= 1e-5
+    # The two differ in the order of their fp32 sums, and in what the 16-bit halves of v then drop: 2^-18 |v| each in
+    # bf16, so 2^-17 sum |v||b| between them, which is at most about 8 times the RMS of y = sum v b for r <= 64.
+    assert rel_err(big[:T].double().cpu().numpy(), y32.double().cpu().numpy()) <= 1e-4
 
 
 def test_few_tokens_with_y_in_the_memory_of_x():
