@@ -63,7 +63,10 @@ def test_few_tokens_in_one_launch(T, N, ranks, dtype, h_in, h_out):
         assert rel_err(c.run(1, y_dtype=torch.float32, flags=L.MID_ROUND).double().cpu().numpy(), c.oracle_delta(1, mid_round=dtype)) <= TOL
     ys = [torch.ones(T, h_out, dtype=c.tdt, device="cuda") for _ in range(2)]
     L.LoraBatch(T, N, h_in, 2).set_ids(c.ids_dev, c.pool).apply([(c.x, y, c.pool) for y in ys], 1)
-    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], (y32 + 1).to(c.tdt))
+    # (twenty items may be past the cluster route: one rounding of y + delta, and the bound derived below)
+    ulp = 2.0 ** (-8 if dtype == "bf16" else -11)
+    assert torch.equal(ys[0], ys[1])
+    assert bool(((ys[0].float() - (y32 + 1)).abs() <= ulp * (y32 + 1).abs() + 1e-4 * y32.pow(2).mean().sqrt()).all())
     reps = 200 // T + 1
     big = torch.zeros(reps * T, h_out, dtype=torch.float32, device="cuda")
     L.LoraBatch(reps * T, N, h_in, 1).set_ids(c.ids_dev.repeat(reps), c.pool).apply([(c.x.repeat(reps, 1), big, c.pool)], 1)
