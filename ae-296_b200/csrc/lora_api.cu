@@ -253,9 +253,8 @@ size_t b200_lora_plan_bytes(int32_t max_tokens, int32_t n_adapters) {
     return plan_words(max_tokens, n_adapters) * 4;
 }
 
-int b200_lora_plan_build(void* plan, size_t plan_bytes, int32_t max_tokens, const void* ids,
-                         int32_t ids_are_i64, int32_t n_tokens, const b200_lora_adapters* adapters,
-                         void* stream) {
+static int plan_build(void* plan, size_t plan_bytes, int32_t max_tokens, const void* ids, int32_t ids_are_i64, int32_t n_tokens,
+                      const b200_lora_adapters* adapters, void* clear, size_t clear_bytes, void* stream) {
     if (!plan || !ids) return B200_LORA_ERR_NULL;
     int rc = check_adapters(adapters);
     if (rc) return rc;
@@ -263,9 +262,15 @@ int b200_lora_plan_build(void* plan, size_t plan_bytes, int32_t max_tokens, cons
     const int cap = max_tokens;
     if (plan_bytes < b200_lora_plan_bytes(cap, adapters->n_adapters)) return B200_LORA_ERR_WORKSPACE;
     if (!aligned16(plan)) return B200_LORA_ERR_ALIGN;
-    cudaError_t e = launch_plan_build(plan, cap, ids, ids_are_i64, n_tokens, plan_adapters(adapters),
+    cudaError_t e = launch_plan_build(plan, cap, ids, ids_are_i64, n_tokens, plan_adapters(adapters), clear, clear_bytes,
                                       static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
+}
+
+int b200_lora_plan_build(void* plan, size_t plan_bytes, int32_t max_tokens, const void* ids,
+                         int32_t ids_are_i64, int32_t n_tokens, const b200_lora_adapters* adapters,
+                         void* stream) {
+    return plan_build(plan, plan_bytes, max_tokens, ids, ids_are_i64, n_tokens, adapters, nullptr, 0, stream);
 }
 
 static int plan_from_segments(void* plan, size_t plan_bytes, int32_t max_tokens, const int32_t* seg_starts, const int32_t* seg_adapter,
@@ -619,11 +624,13 @@ int b200_add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void*
     char* ws = static_cast<char*>(workspace) + pb;
     // Where the control words sit depends on this call's n_tokens and n_adapters, so a buffer that
     // served a call of another shape holds that call's records or partial sums there: clear them
-    // (error word and arrival counters must start at zero) on every call.
-    cudaError_t ce = cudaMemsetAsync(ws, 0, ws_ctl_bytes(n_tokens), static_cast<cudaStream_t>(stream));
-    if (ce != cudaSuccess) return cuda_fail(ce);
-    int rc = b200_lora_plan_build(workspace, pb, n_tokens, indicies, indicies_are_i64, n_tokens, &ad, stream);
-    if (rc) return rc;
+    // (error word and arrival counters must start at zero) on every call.  The plan kernel does that on
+    // its way (a memset node of its own in front of it cost a one-token call 2 us); where no plan is built, a memset.
+    int rc = plan_build(workspace, pb, n_tokens, indicies, indicies_are_i64, n_tokens, &ad, ws, ws_ctl_bytes(n_tokens), stream);
+    if (rc) {
+        cudaError_t ce = cudaMemsetAsync(ws, 0, ws_ctl_bytes(n_tokens), static_cast<cudaStream_t>(stream));
+        return ce == cudaSuccess ? rc : cuda_fail(ce);
+    }
     b200_lora_proj pj;
     pj.x = x; pj.y = y; pj.wa = wa_T_all; pj.wb = wb_T_all;
     pj.ldx = h_in; pj.ldy = h_out; pj.h_in = h_in; pj.h_out = h_out;

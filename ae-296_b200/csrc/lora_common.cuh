@@ -292,7 +292,7 @@ struct PlanAdapters {          // what the plan bakes into its unit records
     int ranks_pow2;               // caller's promise: every rank is 8/16/32/64 (dense: == r_pool)
 };
 cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64, int n_tokens,
-                              const PlanAdapters& ad, cudaStream_t s);
+                              const PlanAdapters& ad, void* clear, size_t clear_bytes, cudaStream_t s);   // `clear`: words to zero
 cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts, const int* seg_adapter,
                                       int n_segs, int n_tokens, int last_end_given, const PlanAdapters& ad, cudaStream_t s);
 cudaError_t launch_bgmv(const ApplyParams& p, int io_dtype, int n_sm, cudaStream_t s);

@@ -7,13 +7,18 @@
 //   tile_tab     128-row tiles of tall runs (>= 32 consecutive rows of one adapter) for the tensor-core kernel
 // It replaces the reference's precomputed index tensor (lightllm/models/lora_gpu.py:120,124)
 // and is integer work only: the tests require it bit-exact against a stable argsort.
+#include <type_traits>
+
 #include "lora_common.cuh"
 
 namespace b200lora {
 
-constexpr int kPlanThreads = 1024;
+// The build is a chain of dependent steps on one CTA, so its time is barriers and scans, not work: a
+// CTA has about as many threads as the batch has tokens (with_plan_threads below).  One warp pays
+// next to nothing for a barrier, 32 warps pay for every one of about sixty.
 
 // exclusive scan of one int per thread over the CTA; returns the prefix, `total` the CTA sum
+template <int NT>
 __device__ int block_scan_excl(int val, int& total, int* warp_sums) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int inc = val;
@@ -26,7 +31,7 @@ __device__ int block_scan_excl(int val, int& total, int* warp_sums) {
     if (lane == 31) warp_sums[wid] = inc;
     __syncthreads();
     if (wid == 0) {
-        int w = warp_sums[lane];
+        int w = lane < NT / 32 ? warp_sums[lane] : 0;
         int winc = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -62,7 +67,7 @@ __device__ __forceinline__ int load_id(const void* ids, int t) {
 }
 
 // Phase A (ids known): histogram, segment table, stable placement.
-template <typename IdT>
+template <typename IdT, int NT>
 __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, int T, int N, int* smem, int* s_cur, int* s_perm) {
     const int tid = threadIdx.x;
     int* warp_sums = smem;              // 33 words
@@ -71,9 +76,9 @@ __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, 
     // histogram, in shared memory when the adapter table fits (hot adapters would serialise
     // hundreds of global atomics on one address)
     int* hist = s_cur ? s_cur : pv.hist;
-    for (int a = tid; a <= N; a += kPlanThreads) hist[a] = 0;
+    for (int a = tid; a <= N; a += NT) hist[a] = 0;
     __syncthreads();
-    for (int t = tid; t < T; t += kPlanThreads) {
+    for (int t = tid; t < T; t += NT) {
         int a = load_id<IdT>(ids, t);
         if (a < 0 || a >= N) *s_bad = 1;
         else atomicAdd(&hist[a], 1);
@@ -85,12 +90,12 @@ __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, 
     }
     // exclusive scan over adapters: token offset and segment index
     int tok_carry = 0, seg_carry = 0;
-    for (int base = 0; base < N; base += kPlanThreads) {
+    for (int base = 0; base < N; base += NT) {
         int a = base + tid;
         int c = a < N ? hist[a] : 0;
         int tot_c, tot_s;
-        int off = block_scan_excl(c, tot_c, warp_sums);
-        int sidx = block_scan_excl(c > 0 ? 1 : 0, tot_s, warp_sums);
+        int off = block_scan_excl<NT>(c, tot_c, warp_sums);
+        int sidx = block_scan_excl<NT>(c > 0 ? 1 : 0, tot_s, warp_sums);
         if (a < N) {
             if (c > 0) {
                 pv.seg_start[seg_carry + sidx] = tok_carry + off;
@@ -114,7 +119,7 @@ __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, 
     // would cost a memory round trip each)
     int* cur = s_cur ? s_cur : pv.hist;
     const int lane = tid & 31, wid = tid >> 5;
-    for (int base = 0; base < T; base += kPlanThreads) {
+    for (int base = 0; base < T; base += NT) {
         int t = base + tid;
         bool valid = t < T;
         int a = valid ? load_id<IdT>(ids, t) : -1 - lane;      // distinct dummies never match
@@ -122,7 +127,7 @@ __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, 
         int rank_in_warp = __popc(peers & ((1u << lane) - 1));
         int leader = __ffs(peers) - 1;
         int cnt = __popc(peers);
-        int n_warps = min(kPlanThreads / 32, (T - base + 31) / 32);
+        int n_warps = min(NT / 32, (T - base + 31) / 32);
         int slot = 0;
         for (int w = 0; w < n_warps; ++w) {
             if (wid == w && valid && lane == leader) {
@@ -149,10 +154,11 @@ __device__ void build_from_ids(PlanView pv, const Scratch& sc, const void* ids, 
 
 // ---- block-wide scans over an array of n ints (shared or global), in place ----------------------
 // inclusive maximum, front to back
+template <int NT>
 __device__ void scan_max_forward(int* arr, int n, int* warp_sums) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int carry = -1;
-    for (int base = 0; base < n; base += kPlanThreads) {
+    for (int base = 0; base < n; base += NT) {
         const int i = base + tid;
         int v = i < n ? arr[i] : -1;
 #pragma unroll
@@ -161,7 +167,7 @@ __device__ void scan_max_forward(int* arr, int n, int* warp_sums) {
         if (lane == 31) warp_sums[wid] = v;
         __syncthreads();
         if (wid == 0) {
-            int w = warp_sums[lane];
+            int w = lane < NT / 32 ? warp_sums[lane] : -1;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w = max(w, t); }
             warp_sums[lane] = w;                            // inclusive maximum over the warps so far
@@ -175,13 +181,14 @@ __device__ void scan_max_forward(int* arr, int n, int* warp_sums) {
     __syncthreads();
 }
 // inclusive minimum, back to front
+template <int NT>
 __device__ void scan_min_backward(int* arr, int n, int* warp_sums) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int kInf = 0x7fffffff;
     int carry = kInf;
-    const int rounds = (n + kPlanThreads - 1) / kPlanThreads;
+    const int rounds = (n + NT - 1) / NT;
     for (int rd = rounds - 1; rd >= 0; --rd) {
-        const int i = rd * kPlanThreads + (kPlanThreads - 1 - tid);     // thread 0 takes the round's last element
+        const int i = rd * NT + (NT - 1 - tid);     // thread 0 takes the round's last element
         int v = i < n ? arr[i] : kInf;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v = min(v, t); }
@@ -189,7 +196,7 @@ __device__ void scan_min_backward(int* arr, int n, int* warp_sums) {
         if (lane == 31) warp_sums[wid] = v;
         __syncthreads();
         if (wid == 0) {
-            int w = warp_sums[lane];
+            int w = lane < NT / 32 ? warp_sums[lane] : kInf;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w = min(w, t); }
             warp_sums[lane] = w;
@@ -218,6 +225,7 @@ __device__ void scan_min_backward(int* arr, int n, int* warp_sums) {
 //   PS(i), PE(i) piece bounds, by the same two scans; the piece's work segments and tiles start at
 //   fixed offsets from PS.
 // t0..t3: four int arrays of T entries (shared memory, or the unit table's room, which is written last).
+template <int NT>
 __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters ad, int* smem, const int* perm, int S,
                             int T, int* t0, int* t1, int* t2, int* t3) {
     const int* ranks = ad.ranks;
@@ -227,9 +235,9 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     int* warp_sums = smem;
     const int kInf = 0x7fffffff;
     // segments: rank (checked against the promise made to the fast kernels), start marks
-    for (int i = tid; i < T; i += kPlanThreads) t0[i] = -1;
+    for (int i = tid; i < T; i += NT) t0[i] = -1;
     __syncthreads();
-    for (int s = tid; s < S; s += kPlanThreads) {
+    for (int s = tid; s < S; s += NT) {
         const int a = sc.seg_adapter[s];
         int r = ranks ? ranks[a] : r_pool;
         if (ad.ranks_pow2 && !((r == 8 || r == 16 || r == 32 || r == 64) && (cum_ranks || r == r_pool)))
@@ -241,16 +249,17 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
         t0[sc.seg_start[s]] = s;
     }
     __syncthreads();
-    scan_max_forward(t0, T, warp_sums);                 // t0 = seg(i)
+    scan_max_forward<NT>(t0, T, warp_sums);                 // t0 = seg(i)
+    if (T >= kTallMin) {
     // run heads
-    for (int i = tid; i < T; i += kPlanThreads) {
+    for (int i = tid; i < T; i += NT) {
         const bool head = i == sc.seg_start[t0[i]] || perm[i] != perm[i - 1] + 1;
         t1[i] = head ? i : -1;
         t2[i] = head ? i : kInf;
     }
     __syncthreads();
-    scan_max_forward(t1, T, warp_sums);                 // t1 = R(i)
-    scan_min_backward(t2, T, warp_sums);                // t2 = first run head >= i
+    scan_max_forward<NT>(t1, T, warp_sums);                 // t1 = R(i)
+    scan_min_backward<NT>(t2, T, warp_sums);                // t2 = first run head >= i
     // tall runs and piece heads; t3 = head flag | tall << 1
     auto tall_at = [&](int i) {
         const int r = sc.seg_rank[t0[i]];
@@ -259,29 +268,37 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
         const int next = i + 1 < T ? min(t2[i + 1], T) : T;         // no further head: the run ends with the batch
         return tile_rank && next - t1[i] >= kTallMin;
     };
-    for (int i = tid; i < T; i += kPlanThreads) {
+    for (int i = tid; i < T; i += NT) {
         const bool seg_head = i == sc.seg_start[t0[i]];
         const bool tall = tall_at(i);
         const bool head = seg_head || (t1[i] == i && (tall || tall_at(i - 1)));
         t3[i] = (head ? 1 : 0) | (tall ? 2 : 0);
     }
     __syncthreads();
-    for (int i = tid; i < T; i += kPlanThreads) {
+    for (int i = tid; i < T; i += NT) {
         const bool head = (t3[i] & 1) != 0;
         t1[i] = head ? i : -1;
         t2[i] = head ? i : kInf;
     }
     __syncthreads();
-    scan_max_forward(t1, T, warp_sums);                 // t1 = PS(i)
-    scan_min_backward(t2, T, warp_sums);                // t2 = first piece head >= i
+    scan_max_forward<NT>(t1, T, warp_sums);                 // t1 = PS(i)
+    scan_min_backward<NT>(t2, T, warp_sums);                // t2 = first piece head >= i
+    } else {                                            // too short for a tall run: the pieces are the segments
+        for (int i = tid; i < T; i += NT) {
+            t1[i] = sc.seg_start[t0[i]];
+            t2[i] = sc.seg_start[t0[i] + 1];
+            t3[i] = 0;
+        }
+        __syncthreads();
+    }
     // work segments and tiles: heads at fixed offsets inside a piece, numbered in position order
     int ws_carry = 0, tile_carry = 0;
-    for (int base = 0; base < T; base += kPlanThreads) {
+    for (int base = 0; base < T; base += NT) {
         const int i = base + tid;
         int wh = 0, th = 0, s = 0, kind = 0, pe = 0;
         if (i < T) {
             const int pb = t1[i];
-            pe = i + 1 < T ? min(t2[i + 1], T) : T;
+            pe = T < kTallMin ? t2[i] : i + 1 < T ? min(t2[i + 1], T) : T;
             const int len = pe - pb, k = i - pb;
             const int ch = (len + kChunkTok - 1) / kChunkTok;
             const int per = (len + ch - 1) / ch;            // balanced chunk length
@@ -291,8 +308,8 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
             th = (kind && (k % kTileM) == 0) ? 1 : 0;
         }
         int tot_w, tot_t;
-        const int w = ws_carry + block_scan_excl(wh, tot_w, warp_sums);
-        const int tile = tile_carry + block_scan_excl(th, tot_t, warp_sums);
+        const int w = ws_carry + block_scan_excl<NT>(wh, tot_w, warp_sums);
+        const int tile = tile_carry + block_scan_excl<NT>(th, tot_t, warp_sums);
         if (wh) {
             sc.ws_start[w] = i;
             sc.ws_adapter[w] = sc.seg_adapter[s];
@@ -329,7 +346,7 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     int tot_short = 0, tot_tall = 0;
     for (int kind = 0; kind < (tot_tiles > 0 ? 2 : 1); ++kind) {
         int carry = kind ? tot_short : 0;
-        for (int base = 0; base < tot_ws; base += kPlanThreads) {
+        for (int base = 0; base < tot_ws; base += NT) {
             const int i = base + tid;
             int w = -1, val = 0;
             if (i < tot_ws) {
@@ -339,7 +356,7 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
                 else w = -1;
             }
             int tot;
-            const int off = block_scan_excl(val, tot, warp_sums);
+            const int off = block_scan_excl<NT>(val, tot, warp_sums);
             if (w >= 0) sc.ws_unit0[w] = carry + off;
             carry += tot;
         }
@@ -354,7 +371,7 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     }
     __syncthreads();
     // unit records: one work segment per thread, n_sub records of four 16-byte stores each
-    for (int i = tid; i < tot_ws; i += kPlanThreads) {
+    for (int i = tid; i < tot_ws; i += NT) {
         const int w = (int)(((long long)i * stride) % tot_ws);
         const int cb = sc.ws_start[w], ce = sc.ws_start[w + 1];
         const int a = sc.ws_adapter[w], r = sc.ws_rank[w] & 0xffff;
@@ -406,9 +423,9 @@ __device__ __forceinline__ void temporaries(PlanView pv, const Scratch& sc, int*
     t0 = base; t1 = base + T; t2 = base + 2 * (size_t)T; t3 = base + 3 * (size_t)T;
 }
 
-template <typename IdT>
-__global__ void __launch_bounds__(kPlanThreads, 1)
-plan_build_kernel(void* plan, int cap, const void* ids, int T, const PlanAdapters ad, int n_cur, int n_perm, int n_scr) {
+template <typename IdT, int NT>
+__global__ void __launch_bounds__(NT, 1)
+plan_build_kernel(void* plan, int cap, const void* ids, int T, const PlanAdapters ad, int n_cur, int n_perm, int n_scr, int* clear, int n_clear) {
     extern __shared__ int dyn_smem[];                      // placement cursors [n_cur], perm [n_perm], working tables
     int* s_cur = n_cur ? dyn_smem : nullptr;
     int* s_perm = n_perm ? dyn_smem + n_cur : nullptr;
@@ -422,17 +439,19 @@ plan_build_kernel(void* plan, int cap, const void* ids, int T, const PlanAdapter
         pv.hdr->error = 0; pv.hdr->cap = cap; pv.hdr->n_adapters = N; pv.hdr->identity = 0;
         pv.hdr->n_units = 0; pv.hdr->n_tiles = 0; pv.hdr->n_units_short = 0; pv.hdr->n_segs = 0; pv.hdr->n_tokens = 0;
     }
+    for (int i = threadIdx.x; i < n_clear; i += NT) clear[i] = 0;       // a workspace's control words, for callers that keep none
     const Scratch sc = make_scratch(pv, dyn_smem, n_cur + n_perm, T, min(T, N), n_scr == 1);
     __syncthreads();
-    build_from_ids<IdT>(pv, sc, ids, T, N, smem, s_cur, s_perm);
+    build_from_ids<IdT, NT>(pv, sc, ids, T, N, smem, s_cur, s_perm);
     __syncthreads();
     if (pv.hdr->error) return;
     int *t0, *t1, *t2, *t3;
     temporaries(pv, sc, dyn_smem + n_cur + n_perm, n_scr, T, t0, t1, t2, t3);
-    build_units(pv, sc, ad, smem, s_perm ? s_perm : pv.perm, smem[42], T, t0, t1, t2, t3);
+    build_units<NT>(pv, sc, ad, smem, s_perm ? s_perm : pv.perm, smem[42], T, t0, t1, t2, t3);
 }
 
-__global__ void __launch_bounds__(kPlanThreads, 1)
+template <int NT>
+__global__ void __launch_bounds__(NT, 1)
 plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_adapter, int S, int T,
                      const PlanAdapters ad, int n_scr, int last_end_given) {
     extern __shared__ int dyn_smem[];                      // working tables, when they fit
@@ -450,7 +469,7 @@ plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_
     }
     __syncthreads();
     // validate: offsets start at 0, end at T, strictly increase; adapters in range
-    for (int s = tid; s < S; s += kPlanThreads) {
+    for (int s = tid; s < S; s += NT) {
         int b = seg_starts[s], e = s + 1 < S || last_end_given ? seg_starts[s + 1] : T, a = seg_adapter[s];
         if (b < 0 || e <= b || e > T) smem[40] = 2;
         if (a < 0 || a >= N) smem[40] = 1;
@@ -460,12 +479,12 @@ plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_
     __syncthreads();
     if (smem[40]) { if (tid == 0) pv.hdr->error = smem[40]; return; }
     const Scratch sc = make_scratch(pv, dyn_smem, 0, T, S, n_scr == 1);
-    for (int s = tid; s < S; s += kPlanThreads) {
+    for (int s = tid; s < S; s += NT) {
         const int b = seg_starts[s], a = seg_adapter[s];
         pv.seg_start[s] = b; pv.seg_adapter[s] = a;
         if (sc.on_chip) { sc.seg_start[s] = b; sc.seg_adapter[s] = a; }
     }
-    for (int t = tid; t < T; t += kPlanThreads) pv.perm[t] = t;
+    for (int t = tid; t < T; t += NT) pv.perm[t] = t;
     if (tid == 0) {
         pv.seg_start[S] = T; pv.hdr->n_segs = S; pv.hdr->n_tokens = T;
         if (sc.on_chip) sc.seg_start[S] = T;
@@ -473,11 +492,36 @@ plan_segments_kernel(void* plan, int cap, const int* seg_starts, const int* seg_
     __syncthreads();
     int *t0, *t1, *t2, *t3;
     temporaries(pv, sc, dyn_smem, n_scr, T, t0, t1, t2, t3);
-    build_units(pv, sc, ad, smem, pv.perm, S, T, t0, t1, t2, t3);
+    build_units<NT>(pv, sc, ad, smem, pv.perm, S, T, t0, t1, t2, t3);
 }
 
+namespace {
+
+// Launches a plan kernel with `smem` bytes of dynamic shared memory (above 48 KB only with the attribute set).
+template <typename... K, typename... A>
+cudaError_t launch_plan(void (*kernel)(K...), int threads, size_t smem, cudaStream_t s, A... args) {
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
+        if (e != cudaSuccess) return e;
+    }
+    kernel<<<1, threads, smem, s>>>(args...);
+    return cudaGetLastError();
+}
+
+// Threads of the plan CTA: a thread per token up to 1024, and enough of them for the adapter table.
+template <typename F>
+cudaError_t with_plan_threads(int n_tokens, int n_adapters, F go) {
+    const int want = n_tokens > n_adapters / 4 ? n_tokens : n_adapters / 4;
+    if (want <= 32) return go(std::integral_constant<int, 32>());
+    if (want <= 128) return go(std::integral_constant<int, 128>());
+    if (want <= 512) return go(std::integral_constant<int, 512>());
+    return go(std::integral_constant<int, 1024>());
+}
+
+}  // namespace
+
 cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64, int n_tokens,
-                              const PlanAdapters& ad, cudaStream_t s) {
+                              const PlanAdapters& ad, void* clear, size_t clear_bytes, cudaStream_t s) {
     // shared-memory copies of the placement cursors and of perm, when they fit
     const int n_cur = (size_t)(ad.n_adapters + 1) * 4 <= 48 * 1024 ? ad.n_adapters + 1 : 0;
     const int n_perm = (size_t)n_tokens * 4 <= 144 * 1024 ? n_tokens : 0;
@@ -489,20 +533,13 @@ cudaError_t launch_plan_build(void* plan, int cap, const void* ids, int ids_i64,
         n_scr = (size_t)(n_cur + n_perm + scr) * 4 <= 200 * 1024 ? 2 : 0;
     }
     const size_t smem = (size_t)(n_cur + n_perm + (n_scr ? scr : 0)) * 4;
-    static bool configured[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(plan_build_kernel<long long>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(plan_build_kernel<int>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    if (ids_i64)
-        plan_build_kernel<long long><<<1, kPlanThreads, smem, s>>>(plan, cap, ids, n_tokens, ad, n_cur, n_perm, n_scr);
-    else
-        plan_build_kernel<int><<<1, kPlanThreads, smem, s>>>(plan, cap, ids, n_tokens, ad, n_cur, n_perm, n_scr);
-    return cudaGetLastError();
+    auto go = [&](auto nt) {
+        int* cw = static_cast<int*>(clear);
+        const int nc = (int)(clear_bytes / 4);
+        if (ids_i64) return launch_plan(plan_build_kernel<long long, nt>, nt, smem, s, plan, cap, ids, n_tokens, ad, n_cur, n_perm, n_scr, cw, nc);
+        return launch_plan(plan_build_kernel<int, nt>, nt, smem, s, plan, cap, ids, n_tokens, ad, n_cur, n_perm, n_scr, cw, nc);
+    };
+    return with_plan_threads(n_tokens, ad.n_adapters, go);
 }
 
 cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts, const int* seg_adapter,
@@ -513,16 +550,11 @@ cudaError_t launch_plan_from_segments(void* plan, int cap, const int* seg_starts
         scr = 4 * (size_t)n_tokens;
         n_scr = scr * 4 <= 200 * 1024 ? 2 : 0;
     }
-    static bool configured[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(plan_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    plan_segments_kernel<<<1, kPlanThreads, n_scr ? scr * 4 : 0, s>>>(plan, cap, seg_starts, seg_adapter, n_segs, n_tokens, ad, n_scr, last_end_given);
-    return cudaGetLastError();
+    const size_t smem = n_scr ? scr * 4 : 0;
+    auto go = [&](auto nt) {
+        return launch_plan(plan_segments_kernel<nt>, nt, smem, s, plan, cap, seg_starts, seg_adapter, n_segs, n_tokens, ad, n_scr, last_end_given);
+    };
+    return with_plan_threads(n_tokens, 1, go);
 }
 
 }  // namespace b200lora
