@@ -12,7 +12,7 @@ import os
 from .build import HOST_PATH, LIB_PATH
 
 F16, BF16, F32 = 0, 1, 2
-MID_ROUND, NO_TENSOR, ONLY_SHRINK, ONLY_EXPAND, DELTA_THEN_ADD, KEEP_PARTIALS = 1, 2, 4, 8, 32, 64
+MID_ROUND, NO_TENSOR, ONLY_SHRINK, ONLY_EXPAND, DELTA_THEN_ADD, KEEP_PARTIALS, OVERWRITE = 1, 2, 4, 8, 32, 64, 128
 MAX_RANK, MAX_PROJ = 64, 4
 
 STATUS = {

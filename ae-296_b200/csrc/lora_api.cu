@@ -357,6 +357,10 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
     if (io_dtype != B200_LORA_F16 && io_dtype != B200_LORA_BF16) return B200_LORA_ERR_DTYPE;
     if (y_dtype != io_dtype && y_dtype != B200_LORA_F32) return B200_LORA_ERR_DTYPE;
     if (layer < 0 || layer >= adapters->n_layers) return B200_LORA_ERR_LAYER;
+    if (flags & B200_LORA_OVERWRITE) {
+        if (tp || (flags & (B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND))) return B200_LORA_ERR_DIM;
+        flags &= ~B200_LORA_DELTA_THEN_ADD;                 // the same on a y of zeros
+    }
     if (!aligned16(plan) || !aligned16(workspace)) return B200_LORA_ERR_ALIGN;
 
     ApplyParams p;
@@ -405,6 +409,41 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
         e = launch_bgmv_cluster(p, io_dtype, s);
         return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
     }
+    bool fast = fast_ranks(adapters);
+    // Dense pools of any other ranks take the TMA kernels' padded form, except where one half runs alone
+    // or the ranks of a group exchange the intermediate (who adds up the split-K slots there works with
+    // the adapters' own ranks).  32 layers of a 93-token decode step, ranks 8 to 64 in R = 64: 3316 us on the
+    // general kernels, 943 us here.
+    const bool padded = !fast && !adapters->packed && !tp && !(flags & (B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND));
+    if (padded) { fast = true; p.flags &= ~B200_LORA_DELTA_THEN_ADD; }   // a flag that these pools do not have
+    for (int i = 0; i < n_proj; ++i)
+        // units are cut at multiples of 128 columns (the shrink kernel's weight box, the widest
+        // per-warp column group of the expand kernel), so the last unit of a row may be partial
+        if ((projs[i].h_in % 128) || (projs[i].h_out % 128) || projs[i].h_in > 8192) fast = false;
+    CUtensorMap bmap[kMaxProj][4];
+    if (fast) {
+        if (padded) memset(bmap, 0, sizeof(bmap));
+        for (int i = 0; i < n_proj && fast; ++i)
+            for (int c = 0; c < 4 && fast; ++c) {
+                const uint32_t rc = 8u << c;
+                if (padded ? rc >= 2u * adapters->r_pool : !adapters->packed && rc != (uint32_t)adapters->r_pool) continue;    // dense pools have one rank
+                if (padded) {
+                    const uint64_t brows = (uint64_t)adapters->n_adapters * adapters->n_layers * projs[i].h_out;
+                    fast = brows <= 0x7fffffffull &&        // box coordinates are 32-bit
+                           tensor_map_2d(&bmap[i][c], projs[i].wb, (uint64_t)adapters->r_pool, brows, rc, 128,
+                                         CU_TENSOR_MAP_SWIZZLE_NONE, 0, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+                }
+                fast = fast && tensor_map_2d(&p.amap[i][c], projs[i].wa, (uint64_t)projs[i].h_in, pool_rows(adapters), 128, rc,
+                                     CU_TENSOR_MAP_SWIZZLE_NONE);
+            }
+    }
+    if (!fast && (p.flags & B200_LORA_OVERWRITE)) {         // the general kernels accumulate only
+        const size_t es = p.y_f32 ? 4 : 2;
+        for (int i = 0; i < n_proj && e == cudaSuccess; ++i)
+            e = cudaMemset2DAsync(projs[i].y, (size_t)projs[i].ldy * es, 0, (size_t)projs[i].h_out * es, (size_t)n_tokens, s);
+        if (e != cudaSuccess) return cuda_fail(e);
+        p.flags &= ~B200_LORA_OVERWRITE;
+    }
     if (!(p.flags & B200_LORA_NO_TENSOR)) {
         SgmvParams sp;
         memset(&sp, 0, sizeof(sp));
@@ -446,34 +485,6 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
                 if (e == cudaSuccess) e = launch_sgmv_tiles(h, sp, io_dtype, n_sm, ts);
             }
         }
-    }
-    bool fast = fast_ranks(adapters);
-    // Dense pools of any other ranks take the TMA kernels' padded form, except where one half runs alone
-    // or the ranks of a group exchange the intermediate (who adds up the split-K slots there works with
-    // the adapters' own ranks).  32 layers of a 93-token decode step, ranks 8 to 64 in R = 64: 3316 us on the
-    // general kernels, 943 us here.
-    const bool padded = !fast && !adapters->packed && !tp && !(flags & (B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND));
-    if (padded) { fast = true; p.flags &= ~B200_LORA_DELTA_THEN_ADD; }   // a flag that these pools do not have
-    for (int i = 0; i < n_proj; ++i)
-        // units are cut at multiples of 128 columns (the shrink kernel's weight box, the widest
-        // per-warp column group of the expand kernel), so the last unit of a row may be partial
-        if ((projs[i].h_in % 128) || (projs[i].h_out % 128) || projs[i].h_in > 8192) fast = false;
-    CUtensorMap bmap[kMaxProj][4];
-    if (fast) {
-        if (padded) memset(bmap, 0, sizeof(bmap));
-        for (int i = 0; i < n_proj && fast; ++i)
-            for (int c = 0; c < 4 && fast; ++c) {
-                const uint32_t rc = 8u << c;
-                if (padded ? rc >= 2u * adapters->r_pool : !adapters->packed && rc != (uint32_t)adapters->r_pool) continue;    // dense pools have one rank
-                if (padded) {
-                    const uint64_t brows = (uint64_t)adapters->n_adapters * adapters->n_layers * projs[i].h_out;
-                    fast = brows <= 0x7fffffffull &&        // box coordinates are 32-bit
-                           tensor_map_2d(&bmap[i][c], projs[i].wb, (uint64_t)adapters->r_pool, brows, rc, 128,
-                                         CU_TENSOR_MAP_SWIZZLE_NONE, 0, CU_TENSOR_MAP_L2_PROMOTION_NONE);
-                }
-                fast = fast && tensor_map_2d(&p.amap[i][c], projs[i].wa, (uint64_t)projs[i].h_in, pool_rows(adapters), 128, rc,
-                                     CU_TENSOR_MAP_SWIZZLE_NONE);
-            }
     }
     auto bgmv = [&](const ApplyParams& q) { return fast ? launch_bgmv_tma(q, padded ? bmap : nullptr, io_dtype, n_sm, s) : launch_bgmv(q, io_dtype, n_sm, s); };
     if (e == cudaSuccess && !tp) e = bgmv(p);

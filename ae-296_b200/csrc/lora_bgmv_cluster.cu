@@ -178,6 +178,7 @@ __device__ __forceinline__ void cluster_expand(const ClusterArgs& p, const ProjA
     constexpr int KS = R == 64 ? 4 : R == 32 ? 2 : 1;
     const int g = lane >> 2, t = lane & 3;
     const int ngrp = u.ntok > 4 ? 2 : 1;
+    const bool overwrite = (p.flags & B200_LORA_OVERWRITE) != 0;      // y counts as zero
     const bool lo_half = (g & 1) != 0;
     unsigned bf[2][KS][2];
 #pragma unroll
@@ -245,11 +246,11 @@ __device__ __forceinline__ void cluster_expand(const ClusterArgs& p, const ProjA
             const long long yoff = (long long)row[grp] * pj.ldy + j0 + jl;
             if (p.y_f32) {
                 float2* yp = reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff);
-                float2 yv = *yp;
+                float2 yv = overwrite ? make_float2(0.f, 0.f) : *yp;
                 yv.x += d0; yv.y += d1;
                 *yp = yv;
             } else {
-                const unsigned yw = *reinterpret_cast<const unsigned*>(ysm + (t + 4 * grp) * ypitch + jl * 2);
+                const unsigned yw = overwrite ? 0u : *reinterpret_cast<const unsigned*>(ysm + (t + 4 * grp) * ypitch + jl * 2);
                 float lo, hi;
                 if (Cvt<T>::is_bf16) {
                     lo = __uint_as_float(yw << 16); hi = __uint_as_float(yw & 0xffff0000u);
@@ -313,7 +314,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     // the same decision in all CTAs of the cluster
     bool live = !hdr.error && seg < hdr.n_wsegs;
     const bool rank_ok = (u.rank == 8 || u.rank == 16 || u.rank == 32 || u.rank == 64) && u.rank <= p.r_cap;
-    if (!hdr.error && (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens || (live && !rank_ok))) {
+    const bool mismatch = !hdr.error && (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens || (live && !rank_ok));
+    if (mismatch) {
         if (tid == 0) atomicMax(err, kErrPlanMismatch);
         live = false;
     }
@@ -321,6 +323,13 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
         cluster_wait();                                    // pairs with the arrival above
         pdl_wait_prior();
         if (tid == 0) pdl_launch_dependents();
+        // nothing applies: the clusters are as many as rows times projections, and each clears its row
+        if ((p.flags & B200_LORA_OVERWRITE) && (hdr.error || mismatch)) {
+            const ProjArgs& pj = p.proj[item - seg * p.n_proj];
+            const int es = p.y_f32 ? 4 : 2;
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<char*>(pj.y) + (long long)seg * pj.ldy * es);
+            for (int q = (int)crank * kThreads + tid; q < pj.h_out * es / 16; q += kCluster * kThreads) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+        }
         return;
     }
     const ProjArgs& pj = p.proj[item - seg * p.n_proj];
@@ -346,7 +355,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     pdl_wait_prior();
     if (tid == 0) pdl_launch_dependents();
     if (warp == 1) {
-        const int y_bytes = p.y_f32 ? 0 : njs * 2;
+        const int y_bytes = p.y_f32 || (p.flags & B200_LORA_OVERWRITE) ? 0 : njs * 2;
         if (lane == 0) { mbar_arrive_expect_tx(bar_a, u.ntok * ncol * 2); mbar_arrive_expect_tx(bar_b, u.ntok * y_bytes); }
         __syncwarp();
         const int q = lane & 7;

@@ -472,7 +472,7 @@ __device__ __forceinline__ void expand_produce(const ApplyParams& p, const PadMa
     const int r = m.rank;
     const int jc = kSuper / n_sub(r);
     const unsigned w_bytes = m.width_ok * r * 2;
-    const unsigned y_bytes = (p.y_f32 || (p.flags & B200_LORA_DELTA_THEN_ADD)) ? 0u : m.width_ok * 2;
+    const unsigned y_bytes = (p.y_f32 || (p.flags & (B200_LORA_DELTA_THEN_ADD | B200_LORA_OVERWRITE))) ? 0u : m.width_ok * 2;
     const bool v_copy = need_v && fc.n_units == 0;
     const unsigned v_bytes = v_copy ? r * 4 : 0u;
     if (parts & 1) {
@@ -649,6 +649,7 @@ __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta&
     const unsigned char* ysb = stage + kWTile;
     constexpr int ypitch = JC * 2 + kYPad;
     const bool staged = !(p.y_f32 || (p.flags & B200_LORA_DELTA_THEN_ADD));
+    const bool overwrite = (p.flags & B200_LORA_OVERWRITE) != 0;      // y counts as zero
     const int jl = jbase + (lo_half ? g + 7 : g);
     const bool col_ok = jbase < m.width_ok;                // the warp's columns lie inside the matrix
     // the staged y values this lane will update, and the rows they go back to
@@ -660,7 +661,7 @@ __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta&
         row[grp] = (grp < ngrp && q < ntok && col_ok) ? tok_rows[q] : -1;
 #pragma unroll
         for (int nb = 0; nb < NBW; ++nb) yw[grp][nb] = 0u;
-        if (staged && row[grp] >= 0) {
+        if (staged && !overwrite && row[grp] >= 0) {
             const unsigned* ys = reinterpret_cast<const unsigned*>(ysb + q * ypitch + jl * 2);
 #pragma unroll
             for (int nb = 0; nb < NBW; ++nb) yw[grp][nb] = ys[nb * 8];
@@ -706,7 +707,7 @@ __device__ __forceinline__ void expand_consume(const ApplyParams& p, const Meta&
             float2* yp = reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff);
             float2 yv[NBW];
 #pragma unroll
-            for (int nb = 0; nb < NBW; ++nb) yv[nb] = yp[nb * 8];
+            for (int nb = 0; nb < NBW; ++nb) yv[nb] = overwrite ? make_float2(0.f, 0.f) : yp[nb * 8];
 #pragma unroll
             for (int nb = 0; nb < NBW; ++nb) {
                 yv[nb].x += d0[nb]; yv[nb].y += d1[nb];
@@ -750,7 +751,10 @@ bgmv_expand_tma_kernel(const __grid_constant__ ApplyParams p, const __grid_const
     PlanView pv = plan_view(p.plan, p.cap, p.n_adapters);
     WorkspaceView ws = workspace_view(p.workspace, p.cap, p.n_proj);
     const PlanHeader hdr = *pv.hdr;
-    if (!plan_usable(hdr, p, &ws.ctl->error)) return;
+    if (!plan_usable(hdr, p, &ws.ctl->error)) {
+        if (p.flags & B200_LORA_OVERWRITE) { pdl_wait_prior(); zero_outputs(p); }
+        return;
+    }
     const int n_units = (p.flags & B200_LORA_NO_TENSOR) ? hdr.n_units : hdr.n_units_short;
     const int n_items = n_units * p.total_super_out;
     const int per_cta = (n_items + (int)gridDim.x - 1) / (int)gridDim.x;

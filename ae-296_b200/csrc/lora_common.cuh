@@ -209,6 +209,19 @@ __device__ __forceinline__ bool plan_usable(const PlanHeader& hdr, const ApplyPa
     return true;
 }
 
+// An apply that applies nothing still defines a y that it is to overwrite: zeros, as a filled y would
+// have kept.  Called by every thread of a grid.
+__device__ __forceinline__ void zero_outputs(const ApplyParams& p) {
+    const int es = p.y_f32 ? 4 : 2;
+    for (int i = 0; i < p.n_proj; ++i) {
+        const int quads = p.proj[i].h_out * es / 16;       // widths are multiples of eight elements
+        for (int row = blockIdx.x; row < p.n_tokens; row += gridDim.x) {
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<char*>(p.proj[i].y) + (long long)row * p.proj[i].ldy * es);
+            for (int q = threadIdx.x; q < quads; q += blockDim.x) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+}
+
 __host__ __device__ __forceinline__ int pad_rank(int r) { return r <= 8 ? 8 : r <= 16 ? 16 : r <= 32 ? 32 : 64; }
 // sub-ranges per 2048-wide super-chunk for a padded rank: 8->4, 16->4, 32->8, 64->16, i.e. a unit is
 // 512 / 512 / 256 / 128 columns (shrink) or rows (expand) wide and holds <= 16 KB of weights

@@ -26,6 +26,8 @@
 // Semantics: the reference's prefill op bmm(bmm(x, A^T), B^T) (lightllm/models/lora_gpu.py:127-128)
 // generalised to adapter-sorted segments; with B200_LORA_MID_ROUND the [T, r] intermediate is
 // rounded to the I/O type exactly as that op's fp16 tensors do.
+#include <initializer_list>
+
 #include "lora_common.cuh"
 
 namespace b200lora {
@@ -230,7 +232,9 @@ __global__ void __launch_bounds__(256) sgmv_ksum_kernel(const __grid_constant__ 
     }
 }
 
-template <typename T>
+// OVER: B200_LORA_OVERWRITE, y counts as zero and nothing of it comes in (a template parameter, since a test of
+// the flag in the epilogue's inner loop cost the accumulating form half a per cent).
+template <typename T, bool OVER>
 __global__ void __launch_bounds__(kSgmvThreads, 1)
 sgmv_tile_kernel(const __grid_constant__ ApplyParams p, const __grid_constant__ SgmvParams sp) {
     extern __shared__ unsigned char smem_raw[];
@@ -396,9 +400,12 @@ sgmv_tile_kernel(const __grid_constant__ ApplyParams p, const __grid_constant__ 
                     if (ny >= (unsigned)nys) retire(ny - nys);
                     if (lane == 0) {
                         const unsigned dst = smem_u32(ystage + ys * kYTile);
-                        mbar_arrive_expect_tx(bar(Y_FULL + ys), kYTile);
-                        tensor_g2s_2d(dst, &sp.ymap[proj], nt * kBN, t.row0, bar(Y_FULL + ys));
-                        tensor_g2s_2d(dst + kYTile / 2, &sp.ymap[proj], nt * kBN + 64, t.row0, bar(Y_FULL + ys));
+                        if (OVER) mbar_arrive(bar(Y_FULL + ys));         // the slot is free
+                        else {
+                            mbar_arrive_expect_tx(bar(Y_FULL + ys), kYTile);
+                            tensor_g2s_2d(dst, &sp.ymap[proj], nt * kBN, t.row0, bar(Y_FULL + ys));
+                            tensor_g2s_2d(dst + kYTile / 2, &sp.ymap[proj], nt * kBN + 64, t.row0, bar(Y_FULL + ys));
+                        }
                         ystate[3 * ys] = t.valid == kBM ? proj : -1;      // other tiles are stored row by row by the epilogue
                         ystate[3 * ys + 1] = nt * kBN;
                         ystate[3 * ys + 2] = t.row0;
@@ -590,7 +597,7 @@ sgmv_tile_kernel(const __grid_constant__ ApplyParams p, const __grid_constant__ 
                                                                    (long long)(t.row0 + row) * pj.ldy + col);
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
-                                float4 y4 = yp[q];
+                                float4 y4 = OVER ? make_float4(0.f, 0.f, 0.f, 0.f) : yp[q];
                                 y4.x += t.scale * v[4 * q]; y4.y += t.scale * v[4 * q + 1];
                                 y4.z += t.scale * v[4 * q + 2]; y4.w += t.scale * v[4 * q + 3];
                                 yp[q] = y4;
@@ -600,7 +607,7 @@ sgmv_tile_kernel(const __grid_constant__ ApplyParams p, const __grid_constant__ 
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
                             uint4* ys4 = reinterpret_cast<uint4*>(ysm + (((2 * c + q) ^ (row & 7)) << 4));
-                            uint4 y4 = *ys4;
+                            uint4 y4 = OVER ? make_uint4(0u, 0u, 0u, 0u) : *ys4;
                             float f[8];
                             Cvt<T>::unpack8(y4, f);
                             y4.x = Cvt<T>::pack2(f[0] + t.scale * v[8 * q], f[1] + t.scale * v[8 * q + 1]);
@@ -641,15 +648,18 @@ cudaError_t launch_sgmv_tiles(const ApplyParams& p, const SgmvParams& sp, int io
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(sgmv_tile_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgmvSmem);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(sgmv_tile_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgmvSmem);
-        if (e != cudaSuccess) return e;
+        for (auto k : {sgmv_tile_kernel<__half, false>, sgmv_tile_kernel<__nv_bfloat16, false>, sgmv_tile_kernel<__half, true>,
+                       sgmv_tile_kernel<__nv_bfloat16, true>}) {
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgmvSmem);
+            if (e != cudaSuccess) return e;
+        }
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
+    const bool over = (p.flags & B200_LORA_OVERWRITE) != 0;
+    auto kernel = io_dtype == B200_LORA_F16 ? (over ? sgmv_tile_kernel<__half, true> : sgmv_tile_kernel<__half, false>)
+                                            : (over ? sgmv_tile_kernel<__nv_bfloat16, true> : sgmv_tile_kernel<__nv_bfloat16, false>);
     auto launch = [&](const ApplyParams& q) {
-        if (io_dtype == B200_LORA_F16) sgmv_tile_kernel<__half><<<n_sm, kSgmvThreads, kSgmvSmem, s>>>(q, sp);
-        else sgmv_tile_kernel<__nv_bfloat16><<<n_sm, kSgmvThreads, kSgmvSmem, s>>>(q, sp);
+        kernel<<<n_sm, kSgmvThreads, kSgmvSmem, s>>>(q, sp);
         return cudaGetLastError();
     };
     // With fewer (tile, projection) pairs than SMs a single launch has to cut every pair by output
@@ -668,9 +678,7 @@ cudaError_t launch_sgmv_tiles(const ApplyParams& p, const SgmvParams& sp, int io
     e = launch_pdl(sgmv_ksum_kernel, dim3(n_sm), dim3(256), 0, s, q, n_sm);
     if (e != cudaSuccess) return e;
     q.flags = p.flags | B200_LORA_ONLY_EXPAND | kFlagLateWait;
-    if (io_dtype == B200_LORA_F16)
-        return launch_pdl(sgmv_tile_kernel<__half>, dim3(n_sm), dim3(kSgmvThreads), kSgmvSmem, s, q, sp);
-    return launch_pdl(sgmv_tile_kernel<__nv_bfloat16>, dim3(n_sm), dim3(kSgmvThreads), kSgmvSmem, s, q, sp);
+    return launch_pdl(kernel, dim3(n_sm), dim3(kSgmvThreads), kSgmvSmem, s, q, sp);
 }
 
 }  // namespace b200lora

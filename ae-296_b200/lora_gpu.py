@@ -125,9 +125,9 @@ class Lora_GPU:
         if bsz in self._decode_stale:
             batch.plan.build(self.select_inds[bsz - 1], self._ad_decode)
             self._decode_stale.discard(bsz)
-        y = torch.zeros(3, bsz, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
+        y = torch.empty(3, bsz, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
         apply([(x, y[i], self._decode_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace,
-              _lib.NO_TENSOR, self._ad_decode)
+              _lib.NO_TENSOR | _lib.OVERWRITE, self._ad_decode)
         return {i: y[i] for i in projs}
 
     def _prefill(self, x, layer_id, projs):
@@ -145,8 +145,8 @@ class Lora_GPU:
             slots = torch.arange(bsz, dtype=torch.int32, device=x.device)
             batch.plan.from_segments(starts, slots, rows, self._ad_prefill)
             self._prefill_shape = (bsz, seqlen)
-        y = torch.zeros(3, rows, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
-        flags = _lib.MID_ROUND if self.prefill_mid_round else 0
+        y = torch.empty(3, rows, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
+        flags = _lib.OVERWRITE | (_lib.MID_ROUND if self.prefill_mid_round else 0)
         x2 = x.reshape(rows, hidden)
         apply([(x2, y[i], self._prefill_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace, flags,
               self._ad_prefill)

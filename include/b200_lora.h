@@ -56,6 +56,10 @@ enum {
     B200_LORA_KEEP_PARTIALS = 64, /* with B200_LORA_ONLY_SHRINK on the TMA kernels: leave the split-K partial sums
                                    as they are instead of adding them up into v (a caller that reduces them
                                    itself, or that times the shrink kernel alone) */
+    B200_LORA_OVERWRITE = 128, /* y = delta instead of y += delta, for callers whose y would start at zero: y is
+                                   neither filled nor read.  An apply that applies nothing (a plan whose build
+                                   failed, or of another size) writes zeros.  Not for b200_lora_apply_tp and
+                                   not with B200_LORA_ONLY_SHRINK / B200_LORA_ONLY_EXPAND (ERR_DIM) */
     B200_LORA_DELTA_THEN_ADD = 32 /* 16-bit y only: round the delta to the I/O type and add it to y in that
                                    type, as the reference's `q += q_lora` does
                                    (lightllm/models/llama/layer_infer/transformer_layer_infer.py:160-170).

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import ae296_b200 as L
+from ae296_b200 import _lib
 from lora_testlib import TOL, Case, rel_err
 from oracle import lora_oracle as O
 
@@ -276,3 +277,38 @@ def test_adapter_swapped_in_on_a_side_stream():
     assert torch.equal(after[rows], before[rows])           # other adapters' tokens are untouched
     with pytest.raises(ValueError):
         c.pool.load_adapter_async(a, A_new[:, :8], B_new, side)
+
+
+@pytest.mark.parametrize("kind", ["cluster", "streaming", "padded", "general", "tiles", "tiles_many"])
+@pytest.mark.parametrize("y_dtype", [None, torch.float32])
+def test_overwrite_equals_accumulating_into_zeros(kind, y_dtype):
+    """OVERWRITE on every route: the bits that a zero-filled y gets, whatever y held; nothing outside the rows;
+    zeros where the plan applies nothing."""
+    T, h = {"cluster": (5, 512), "streaming": (90, 512), "padded": (90, 512), "general": (40, 328), "tiles": (300, 512),
+            "tiles_many": (5000, 512)}[kind]
+    ids = np.random.default_rng(T).integers(0, 6, T)
+    if kind.startswith("tiles"):
+        ids = np.sort(ids)
+        ids[-7:] = np.arange(7) % 6                                # a few rows for the decode kernels too
+    ranks = np.array([3, 12, 20, 33, 50, 64] if kind == "padded" else [8, 16, 32, 64, 16, 32], np.int32)
+    c = Case(T, 6, h, h, ranks, "fp16", dense=kind == "padded", seed=T, ids=ids, n_layers=1)
+    flags = _lib.OVERWRITE
+    yt = c.tdt if y_dtype is None else y_dtype
+    batch = L.LoraBatch(T, 6, h, 1).set_ids(c.ids_dev, c.pool, tiles=kind.startswith("tiles"))
+    want = torch.zeros(T, h, dtype=yt, device="cuda")
+    batch.apply([(c.x, want, c.pool)], 0)
+    big = torch.full((T + 2, h + 16), float("nan"), dtype=yt, device="cuda")
+    got = big[1:-1, 8:8 + h]
+    batch.apply([(c.x, got, c.pool)], 0, flags)
+    batch.workspace.check()
+    assert torch.equal(got, want)
+    assert bool(torch.isnan(big[0]).all()) and bool(torch.isnan(big[-1]).all())
+    assert bool(torch.isnan(big[:, :8]).all()) and bool(torch.isnan(big[:, 8 + h:]).all())
+    bad = c.ids_dev.clone()
+    bad[T // 2] = 6                                                # no such adapter: the plan applies nothing
+    batch.set_ids(bad, c.pool, tiles=kind.startswith("tiles"))
+    got.fill_(float("nan"))
+    batch.apply([(c.x, got, c.pool)], 0, flags)
+    torch.cuda.synchronize()
+    assert bool((got == 0).all())
+    assert bool(torch.isnan(big[0]).all()) and bool(torch.isnan(big[:, 8 + h:]).all())
