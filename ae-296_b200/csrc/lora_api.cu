@@ -341,13 +341,14 @@ static bool tp_usable(const b200_lora_tp* tp) {
     return true;
 }
 
-// One apply.  With `tp` it is the tensor-parallel form: each chain (the tiles on the side stream,
+// One apply.  With `direct_ids` the plan buffer holds no plan: the cluster kernel works from the ids, or
+// nothing is launched (B200_LORA_ERR_UNSUPPORTED).  With `tp` it is the tensor-parallel form: each chain (the tiles on the side stream,
 // the BGMV kernels on the caller's) runs its shrink half, the exchange of its own rows of v over
 // the ranks, and its expand half.
 static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lora_adapters* adapters,
                       const void* plan, int32_t max_tokens, int32_t n_tokens, int32_t layer, int32_t io_dtype,
                       int32_t y_dtype, int32_t flags, void* workspace, size_t workspace_bytes_, void* stream,
-                      const b200_lora_tp* tp, int skip_arrival) {
+                      const b200_lora_tp* tp, int skip_arrival, const void* direct_ids = nullptr, int direct_i64 = 0) {
     if (!projs || !plan || !workspace) return B200_LORA_ERR_NULL;
     if (tp && !tp_usable(tp)) return B200_LORA_ERR_DIM;
     if (tp && (flags & (B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND))) return B200_LORA_ERR_DIM;
@@ -406,9 +407,10 @@ static int apply_core(const b200_lora_proj* projs, int32_t n_proj, const b200_lo
     // a batch shorter than the shortest tall run has none: no tile launches, no side stream
     if (!sgmv_tiles_supported(p) || n_tokens < kTallMin) p.flags |= B200_LORA_NO_TENSOR;
     if (!tp && cluster_route(p, adapters, io_dtype)) {
-        e = launch_bgmv_cluster(p, io_dtype, s);
+        e = launch_bgmv_cluster(p, direct_ids, direct_i64, io_dtype, s);
         return e == cudaSuccess ? B200_LORA_OK : cuda_fail(e);
     }
+    if (direct_ids) return B200_LORA_ERR_UNSUPPORTED;       // every other route needs a plan
     bool fast = fast_ranks(adapters);
     // Dense pools of any other ranks take the TMA kernels' padded form, except where one half runs alone
     // or the ranks of a group exchange the intermediate (who adds up the split-K slots there works with
@@ -620,11 +622,11 @@ size_t b200_add_lora_bgmv_workspace_bytes(int32_t n_tokens, int32_t n_adapters, 
     return ((pb + 255) & ~size_t(255)) + wb;
 }
 
-int b200_add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void* wb_T_all,
+static int add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void* wb_T_all,
                        const void* indicies, int32_t indicies_are_i64, int32_t n_tokens,
                        int32_t h_in, int32_t h_out, int32_t n_adapters, int32_t n_layers, int32_t r,
                        int32_t layer_idx, float scale, int32_t dtype,
-                       void* workspace, size_t workspace_bytes_, void* stream) {
+                       void* workspace, size_t workspace_bytes_, void* stream, bool plan_wanted) {
     if (!workspace) return B200_LORA_ERR_NULL;
     if (n_tokens < 1 || n_adapters < 1) return B200_LORA_ERR_DIM;
     if (workspace_bytes_ < b200_add_lora_bgmv_workspace_bytes(n_tokens, n_adapters, h_in)) return B200_LORA_ERR_WORKSPACE;
@@ -633,6 +635,16 @@ int b200_add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void*
     ad.n_adapters = n_adapters; ad.n_layers = n_layers; ad.r_pool = r; ad.packed = 0; ad.scale = scale;
     size_t pb = (b200_lora_plan_bytes(n_tokens, n_adapters) + 255) & ~size_t(255);
     char* ws = static_cast<char*>(workspace) + pb;
+    b200_lora_proj pj;
+    pj.x = x; pj.y = y; pj.wa = wa_T_all; pj.wb = wb_T_all;
+    pj.ldx = h_in; pj.ldy = h_out; pj.h_in = h_in; pj.h_out = h_out;
+    // A few tokens whose plan nobody will read: no plan kernel (a one-token call: 12.3 us with it, 4.5 without).
+    // Whatever stands against that, a refused argument included, is the longer way's to report.
+    if (!plan_wanted && indicies && n_tokens <= kDirectTokens) {
+        int rc = apply_core(&pj, 1, &ad, workspace, n_tokens, n_tokens, layer_idx, dtype, dtype, B200_LORA_NO_TENSOR, ws,
+                            workspace_bytes_ - pb, stream, nullptr, 0, indicies, indicies_are_i64);
+        if (rc == B200_LORA_OK || rc == B200_LORA_ERR_CUDA) return rc;
+    }
     // Where the control words sit depends on this call's n_tokens and n_adapters, so a buffer that
     // served a call of another shape holds that call's records or partial sums there: clear them
     // (error word and arrival counters must start at zero) on every call.  The plan kernel does that on
@@ -642,11 +654,17 @@ int b200_add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void*
         cudaError_t ce = cudaMemsetAsync(ws, 0, ws_ctl_bytes(n_tokens), static_cast<cudaStream_t>(stream));
         return ce == cudaSuccess ? rc : cuda_fail(ce);
     }
-    b200_lora_proj pj;
-    pj.x = x; pj.y = y; pj.wa = wa_T_all; pj.wb = wb_T_all;
-    pj.ldx = h_in; pj.ldy = h_out; pj.h_in = h_in; pj.h_out = h_out;
     return b200_lora_apply(&pj, 1, &ad, workspace, n_tokens, n_tokens, layer_idx, dtype, dtype, B200_LORA_NO_TENSOR, ws,
                            workspace_bytes_ - pb, stream);
+}
+
+int b200_add_lora_bgmv(void* y, const void* x, const void* wa_T_all, const void* wb_T_all,
+                       const void* indicies, int32_t indicies_are_i64, int32_t n_tokens,
+                       int32_t h_in, int32_t h_out, int32_t n_adapters, int32_t n_layers, int32_t r,
+                       int32_t layer_idx, float scale, int32_t dtype,
+                       void* workspace, size_t workspace_bytes_, void* stream) {
+    return add_lora_bgmv(y, x, wa_T_all, wb_T_all, indicies, indicies_are_i64, n_tokens, h_in, h_out, n_adapters, n_layers, r,
+                         layer_idx, scale, dtype, workspace, workspace_bytes_, stream, true);
 }
 
 // ---- allocation-free variant ---------------------------------------------------------------
@@ -672,9 +690,9 @@ int b200_add_lora_bgmv_static(void* y, const void* x, const void* wa_T_all, cons
         cudaGetDevice(&dev);
         g_static_last_pb[dev] = pb;              // where the last call's workspace part begins
     }
-    return b200_add_lora_bgmv(y, x, wa_T_all, wb_T_all, indicies, indicies_are_i64, n_tokens, h_in, h_out,
-                              n_adapters, n_layers, r, layer_idx, scale, dtype, scratch,
-                              (size_t)B200_LORA_STATIC_SCRATCH_BYTES, stream);
+    return add_lora_bgmv(y, x, wa_T_all, wb_T_all, indicies, indicies_are_i64, n_tokens, h_in, h_out,
+                         n_adapters, n_layers, r, layer_idx, scale, dtype, scratch,
+                         (size_t)B200_LORA_STATIC_SCRATCH_BYTES, stream, false);
 }
 
 int b200_add_lora_bgmv_static_status(void* stream) {

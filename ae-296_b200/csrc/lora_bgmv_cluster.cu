@@ -52,6 +52,10 @@ struct ClusterArgs {
     int n_proj, n_adapters, n_layers, r_pool, packed, layer, flags, y_f32, cap, n_tokens;
     int r_cap;                 // largest rank the shared memory was sized for
     int kcols, jcols;          // widest slice of h_in and of h_out
+    // DIRECT: the adapter of each token instead of a plan (one projection, dense pool of one rank)
+    const void* ids;
+    int ids_i64;
+    float scale;
 };
 
 // Shared memory of one CTA: byte offsets of its parts.
@@ -288,7 +292,37 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs& p, const ProjArg
     cluster_expand<T, R>(p, pj, u, smem + l.b, smem + l.y, l.ypitch, vt, j0, njs, lane, warp);
 }
 
-template <typename T>
+// The work segments of a call that has no plan, for at most kDirectTokens tokens: token t heads one when it is
+// the 1st, 9th, ... token of its adapter, and the segment is that token and the next seven of the adapter (a
+// plan would cut in the same number of pieces and balance their lengths).  Every warp works it out from the
+// ids.  Returns whether t heads a segment; `bad` when any id names no adapter.
+__device__ __forceinline__ bool direct_segment(const ClusterArgs& p, int t, int lane, UnitRec& u, bool& bad) {
+    int id[2];
+    bool in[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        in[h] = i < p.n_tokens;
+        id[h] = !in[h] ? -1 : p.ids_i64 ? (int)reinterpret_cast<const long long*>(p.ids)[i] : reinterpret_cast<const int*>(p.ids)[i];
+    }
+    bad = __ballot_sync(0xffffffffu, (in[0] && (id[0] < 0 || id[0] >= p.n_adapters)) || (in[1] && (id[1] < 0 || id[1] >= p.n_adapters))) != 0;
+    const int a0 = __shfl_sync(0xffffffffu, id[0], t & 31), a1 = __shfl_sync(0xffffffffu, id[1], t & 31);
+    const int a = t < 32 ? a0 : a1;
+    unsigned long long m = __ballot_sync(0xffffffffu, in[0] && id[0] == a);
+    m |= (unsigned long long)__ballot_sync(0xffffffffu, in[1] && id[1] == a) << 32;
+    const int before = __popcll(m & ((1ull << t) - 1));
+    m = m >> t << t;
+    u.adapter = a; u.rank = p.r_pool; u.sub = 0; u.ntok = (short)min(8, __popcll(m)); u.scale = p.scale; u.wseg = t; u.start = t;
+    u.cum_lo = u.cum_hi = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        u.tok[i] = m ? __ffsll((long long)m) - 1 : t;
+        m &= m - 1;
+    }
+    return (before & 7) == 0;
+}
+
+template <typename T, bool DIRECT>
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgmv_cluster_kernel(const __grid_constant__ ClusterArgs p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -300,10 +334,27 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     unsigned* err = &reinterpret_cast<WorkspaceCtl*>(p.workspace)->error;
     // header and segment record in one round trip (the record of a segment the plan does not have is not used)
     UnitRec u;
+    PlanHeader hdr;
+    bool heads = true;
+    if constexpr (DIRECT) {
+        pdl_wait_prior();                                  // the ids may come from the predecessor
+        if (tid == 0) pdl_launch_dependents();
+        bool bad;
+        heads = direct_segment(p, seg, lane, u, bad);
+        hdr.error = bad ? 1 : 0;
+        hdr.cap = p.cap; hdr.n_tokens = hdr.n_wsegs = p.n_tokens;
+        // What the status call reads.  All clusters start together, and a wait takes seconds to expire, so no
+        // other CTA's record can be older than this.
+        if (blockIdx.x == 0 && tid == 0) {
+            pv.hdr->error = hdr.error;
+            *err = 0u;
+        }
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        reinterpret_cast<uint4*>(&u)[i] = __ldg(reinterpret_cast<const uint4*>(pv.seg_tab + (size_t)seg * 16) + i);
-    const PlanHeader hdr = *pv.hdr;
+        for (int i = 0; i < 4; ++i)
+            reinterpret_cast<uint4*>(&u)[i] = __ldg(reinterpret_cast<const uint4*>(pv.seg_tab + (size_t)seg * 16) + i);
+        hdr = *pv.hdr;
+    }
     const unsigned bar_a = smem_u32(smem + l.bars), bar_b = bar_a + 8;
     if (tid == 0) {
         mbar_init(bar_a, 2);                               // weights, and x
@@ -312,7 +363,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     }
     __syncthreads();
     // the same decision in all CTAs of the cluster
-    bool live = !hdr.error && seg < hdr.n_wsegs;
+    bool live = !hdr.error && seg < hdr.n_wsegs && heads;
     const bool rank_ok = (u.rank == 8 || u.rank == 16 || u.rank == 32 || u.rank == 64) && u.rank <= p.r_cap;
     const bool mismatch = !hdr.error && (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens || (live && !rank_ok));
     if (mismatch) {
@@ -359,7 +410,10 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
         if (lane == 0) { mbar_arrive_expect_tx(bar_a, u.ntok * ncol * 2); mbar_arrive_expect_tx(bar_b, u.ntok * y_bytes); }
         __syncwarp();
         const int q = lane & 7;
-        const int tok = __ldg(pv.seg_tab + (size_t)seg * 16 + 8 + q);
+        int tok = u.tok[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i)
+            if (q == i) tok = u.tok[i];
         if (q < u.ntok) {
             if (lane < 8 && ncol > 0)
                 bulk_g2s(sbase + l.x + q * l.pitch, reinterpret_cast<const T*>(pj.x) + (long long)tok * pj.ldx + k0, ncol * 2, bar_a);
@@ -400,8 +454,9 @@ int resident_clusters(int smem) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaFuncSetAttribute(bgmv_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, bgmv_cluster_kernel<T>, &cfg) != cudaSuccess) {
+    if (cudaFuncSetAttribute(bgmv_cluster_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(bgmv_cluster_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, bgmv_cluster_kernel<T, false>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         n = 0;                                             // the apply stays on the streaming kernels
     }
@@ -434,7 +489,7 @@ int bgmv_cluster_limit(const ApplyParams& p, int io_dtype) {
     return io_dtype == B200_LORA_F16 ? resident_clusters<__half>(smem) : resident_clusters<__nv_bfloat16>(smem);
 }
 
-cudaError_t launch_bgmv_cluster(const ApplyParams& p, int io_dtype, cudaStream_t s) {
+cudaError_t launch_bgmv_cluster(const ApplyParams& p, const void* ids, int ids_i64, int io_dtype, cudaStream_t s) {
     ClusterArgs a;
     memset(&a, 0, sizeof(a));
     a.r_cap = pad_rank(p.r_pool);
@@ -449,7 +504,9 @@ cudaError_t launch_bgmv_cluster(const ApplyParams& p, int io_dtype, cudaStream_t
     const int smem = layout_of(a.r_cap, a.kcols, a.jcols).total;
     // a cluster per (work segment, projection); there are at most as many segments as tokens
     const int n = p.n_tokens * p.n_proj;
-    auto kernel = io_dtype == B200_LORA_F16 ? bgmv_cluster_kernel<__half> : bgmv_cluster_kernel<__nv_bfloat16>;
+    a.ids = ids; a.ids_i64 = ids_i64; a.scale = p.scale;
+    auto kernel = io_dtype == B200_LORA_F16 ? bgmv_cluster_kernel<__half, false> : bgmv_cluster_kernel<__nv_bfloat16, false>;
+    if (ids) kernel = io_dtype == B200_LORA_F16 ? bgmv_cluster_kernel<__half, true> : bgmv_cluster_kernel<__nv_bfloat16, true>;
     return launch_pdl(kernel, dim3(n * kCluster), dim3(kThreads), smem, s, a);
 }
 

@@ -315,7 +315,10 @@ int bgmv_tma_shrink_grid(int n_sm);       // CTAs of the TMA shrink kernel (whoe
 // one launch per apply for a few tokens (a thread-block cluster per work segment and projection)
 bool bgmv_cluster_fits(const ApplyParams& p);     // widths and shared memory
 int bgmv_cluster_limit(const ApplyParams& p, int io_dtype);      // clusters of this size that run at once
-cudaError_t launch_bgmv_cluster(const ApplyParams& p, int io_dtype, cudaStream_t s);
+// `ids` (else NULL): no plan, the kernel finds the segments of these at most kDirectTokens tokens itself; one
+// projection, dense pool of one rank
+constexpr int kDirectTokens = 64;
+cudaError_t launch_bgmv_cluster(const ApplyParams& p, const void* ids, int ids_i64, int io_dtype, cudaStream_t s);
 cudaError_t launch_tp_exchange(const b200_lora_tp* tp, void* workspace, int n_proj, int cap, int n_tokens, int skip_push,
                                int n_sm, cudaStream_t s);
 // one exchange of a tensor-parallel apply: the rows of the plan's tiles (`tall`) or of its BGMV work segments

@@ -65,3 +65,23 @@ def test_static_scratch_entry_point_matches_workspace_entry_point_twice():
     with pytest.raises(L.LoraError) as e:
         L.add_lora_bgmv_static_status()
     assert e.value.code == -8
+
+
+@pytest.mark.parametrize("t,n", [(1, 1), (9, 1), (17, 2), (24, 24), (40, 3)])
+@pytest.mark.parametrize("ids_dtype", [torch.int32, torch.int64])
+def test_static_call_without_a_plan_matches_the_planned_one(t, n, ids_dtype):
+    """Few tokens: the kernel finds the segments in the ids itself, one to eight tokens each, with tokens of an
+    adapter in both halves of a warp's view.  A bad id applies nothing, and the next good call clears its record."""
+    x, wa, wb, ids, y0 = _inputs(500 + t, t, n, 1024, 640, 16, torch.float16)
+    ids = ids.to(ids_dtype)
+    want, got = y0.clone(), y0.clone()
+    ws = torch.empty(L.add_lora_bgmv_workspace_bytes(t, n, 1024), dtype=torch.uint8, device="cuda")
+    L.add_lora_bgmv_once(want, x, wa, wb, ids, 1, 0.5, ws)
+    bad = ids.clone()
+    bad[-1] = n
+    for call_ids, expect in ((bad, y0), (ids, want)):
+        got = y0.clone()
+        L.add_lora_bgmv_static(got, x, wa, wb, call_ids, 1, 0.5)
+        torch.cuda.synchronize()
+        assert torch.equal(got, expect)
+    L.add_lora_bgmv_static_status()
