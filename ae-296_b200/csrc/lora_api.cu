@@ -167,7 +167,7 @@ bool fast_ranks(const b200_lora_adapters* ad) {
 //   h 4096, r 16 (3 CTAs an SM):  1 item 5.5 / 3.6   24 items 7.6 / 4.7   48 items 8.8 / 7.4   64 items 9.7 / 10.5
 //   h 4096, r 64 (1 CTA an SM):   1 item 6.8 / 5.0   12 items 9.5 / 6.9   16 items 10.4 / 11.9
 //   h 2048, r 64 (2 CTAs an SM):  1 item 6.1 / 4.7   24 items 9.1 / 6.8   32 items 9.9 / 8.3   36 items 10.2 / 11.7
-// and bgmv_cluster_limit() is 48 to 54, 14 to 18 and 28 to 36 there.
+// bgmv_cluster_limit() is 48 in the first row and falls with the CTAs that fit an SM.
 bool cluster_route(const ApplyParams& p, const b200_lora_adapters* ad, int io_dtype) {
     if ((long long)p.n_tokens * p.n_proj > 1024) return false;       // far beyond any limit
     const int other = B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND | B200_LORA_DELTA_THEN_ADD;
