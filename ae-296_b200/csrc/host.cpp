@@ -9,8 +9,13 @@
 // The functions take the short path only: operands that are exactly what the ops document.  Anything else
 // (a wrong shape or type, a table that has to grow) returns kSlow and the Python code beside the call
 // raises the error or prepares what is missing.  The GIL is given up around the CUDA calls.
+//
+// Reading a tensor can throw (one without storage, as under vmap or in a tracer; a driver that is not usable):
+// every entry point turns that into the Python exception the same access raises in Python, and no tensor is
+// touched while the GIL is given up.
 #include <Python.h>
 
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
@@ -127,6 +132,18 @@ PyObject* slow() {                 // an attribute or conversion error on the sh
     return PyLong_FromLong(kSlow);
 }
 
+// An entry point whose C++ exceptions become Python exceptions.
+using FastCall = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
+template <FastCall F>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+    try {
+        return F(self, args, nargs);
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+
 // apply(projs, plan, layer, workspace, flags, adapters | None) -> status
 PyObject* py_apply(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (nargs != 6) return slow();
@@ -188,11 +205,13 @@ PyObject* py_plan_build(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!ids.is_cuda() || !ids.is_contiguous() || (ids.scalar_type() != at::kInt && ids.scalar_type() != at::kLong)) return slow();
     const int64_t n = ids.numel();
     Ref num(PyLong_FromLongLong(n));
-    if (!num || PyObject_SetAttr(args[0], s_n_tokens, num.o) != 0) return slow();
     void* stream = stream_of(ids);
+    const void* ids_ptr = ids.data_ptr();
+    const int is_i64 = ids.scalar_type() == at::kLong;
+    if (!num || PyObject_SetAttr(args[0], s_n_tokens, num.o) != 0) return slow();
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = b200_lora_plan_build(plan.buf, plan.nbytes, plan.max_tokens, ids.data_ptr(), ids.scalar_type() == at::kLong, (int32_t)n, &ad, stream);
+    rc = b200_lora_plan_build(plan.buf, plan.nbytes, plan.max_tokens, ids_ptr, is_i64, (int32_t)n, &ad, stream);
     Py_END_ALLOW_THREADS
     return PyLong_FromLong(rc);
 }
@@ -210,10 +229,10 @@ PyObject* py_plan_segments(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         return slow();
     const int64_t n = owner.numel(), t = PyLong_AsLongLong(args[3]);
     if (PyErr_Occurred() || starts.numel() < n) return slow();
-    if (PyObject_SetAttr(args[0], s_n_tokens, args[3]) != 0) return slow();
     void* stream = stream_of(starts);
     const bool ends = starts.numel() > n;
     const int32_t *sp = static_cast<const int32_t*>(starts.data_ptr()), *op = static_cast<const int32_t*>(owner.data_ptr());
+    if (PyObject_SetAttr(args[0], s_n_tokens, args[3]) != 0) return slow();
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = (ends ? b200_lora_plan_from_segments : b200_lora_plan_from_requests)(plan.buf, plan.nbytes, plan.max_tokens, sp, op, (int32_t)n,
@@ -354,21 +373,23 @@ PyObject* py_bgmv_static(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     OpArgs a;
     if (nargs != 7 || !read_op(args, a)) return slow();
     void* stream = stream_of(*a.x);
+    void* y = a.y->data_ptr();
+    const void *x = a.x->data_ptr(), *wa = a.wa->data_ptr(), *wb = a.wb->data_ptr(), *ids = a.ids->data_ptr();
+    const int is_i64 = a.ids->scalar_type() == at::kLong;
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = b200_add_lora_bgmv_static(a.y->data_ptr(), a.x->data_ptr(), a.wa->data_ptr(), a.wb->data_ptr(), a.ids->data_ptr(),
-                                   a.ids->scalar_type() == at::kLong, (int32_t)a.t, (int32_t)a.h_in, (int32_t)a.h_out, (int32_t)a.n,
+    rc = b200_add_lora_bgmv_static(y, x, wa, wb, ids, is_i64, (int32_t)a.t, (int32_t)a.h_in, (int32_t)a.h_out, (int32_t)a.n,
                                    (int32_t)a.l, (int32_t)a.r, (int32_t)a.layer, (float)a.scale, a.io, stream);
     Py_END_ALLOW_THREADS
     return PyLong_FromLong(rc);
 }
 
 PyMethodDef kMethods[] = {
-    {"apply", (PyCFunction)(void*)py_apply, METH_FASTCALL, nullptr},
-    {"plan_build", (PyCFunction)(void*)py_plan_build, METH_FASTCALL, nullptr},
-    {"plan_segments", (PyCFunction)(void*)py_plan_segments, METH_FASTCALL, nullptr},
-    {"bgmv", (PyCFunction)(void*)py_bgmv, METH_FASTCALL, nullptr},
-    {"bgmv_static", (PyCFunction)(void*)py_bgmv_static, METH_FASTCALL, nullptr},
+    {"apply", (PyCFunction)(void*)guarded<py_apply>, METH_FASTCALL, nullptr},
+    {"plan_build", (PyCFunction)(void*)guarded<py_plan_build>, METH_FASTCALL, nullptr},
+    {"plan_segments", (PyCFunction)(void*)guarded<py_plan_segments>, METH_FASTCALL, nullptr},
+    {"bgmv", (PyCFunction)(void*)guarded<py_bgmv>, METH_FASTCALL, nullptr},
+    {"bgmv_static", (PyCFunction)(void*)guarded<py_bgmv_static>, METH_FASTCALL, nullptr},
     {"bgmv_register", py_bgmv_register, METH_VARARGS, nullptr},
     {"bgmv_forget", py_bgmv_forget, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
