@@ -242,42 +242,46 @@ PyObject* py_plan_segments(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 // ---- the reference's operator call ---------------------------------------------------------------
-// Plan and workspace behind add_lora_bgmv for one (device, stream): the memory belongs to the Python side,
-// which registers it here; what the plan was built from is kept here.  The index tensor is held weakly:
-// its object stays comparable by address, its storage does not stay alive.
+// Plan and workspace behind add_lora_bgmv for one (device, stream, graph capture): the memory belongs to the
+// Python side, which registers it here; what the plan was built from is kept here.  A capture has an entry of
+// its own, since every replay writes the plan again: an eager call must not find its plan replaced by a replay.
+// The index tensor is held weakly: its object stays comparable by address, its storage does not stay alive.
 struct OpEntry {
-    void* stream;
-    int device;
-    void *plan, *ws;
-    size_t plan_bytes, ws_bytes;
-    int cap_t, cap_n, cap_h;
-    bool built;
-    c10::weak_intrusive_ptr<c10::TensorImpl> ids;
-    const void* ids_ptr;
-    uint32_t version;
-    int ids_type, t, n, r;
-    float scale;
-    unsigned long long capture;
-    OpEntry() : stream(nullptr), device(-1), plan(nullptr), ws(nullptr), plan_bytes(0), ws_bytes(0), cap_t(0), cap_n(0), cap_h(0), built(false),
-                ids(c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()), ids_ptr(nullptr), version(0), ids_type(0), t(0), n(0), r(0),
-                scale(0.f), capture(0) {}
+    void* stream = nullptr;
+    int device = -1;
+    unsigned long long capture = 0;
+    void *plan = nullptr, *ws = nullptr;
+    size_t plan_bytes = 0, ws_bytes = 0;
+    int cap_t = 0, cap_n = 0, cap_h = 0;
+    bool built = false;
+    c10::weak_intrusive_ptr<c10::TensorImpl> ids{c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()};
+    const void* ids_ptr = nullptr;
+    uint32_t version = 0;
+    int ids_type = 0, t = 0, n = 0, r = 0;
+    float scale = 0.f;
 };
 std::vector<OpEntry>* g_ops;       // guarded by the GIL; a process has a handful of streams
 
-OpEntry* find_op(void* stream, int device) {
+OpEntry* find_op(void* stream, int device, unsigned long long capture) {
     for (OpEntry& e : *g_ops)
-        if (e.stream == stream && e.device == device) return &e;
+        if (e.stream == stream && e.device == device && e.capture == capture) return &e;
     return nullptr;
 }
 
-// bgmv_register(stream, device, plan_ptr, plan_bytes, ws_ptr, ws_bytes, cap_t, cap_n, cap_h)
+// bgmv_register(stream, device, capture, plan_ptr, plan_bytes, ws_ptr, ws_bytes, cap_t, cap_n, cap_h)
+// A stream is in one capture at a time: entries of its earlier captures go.
 PyObject* py_bgmv_register(PyObject*, PyObject* args) {
-    unsigned long long stream, plan, ws, plan_bytes, ws_bytes;
+    unsigned long long stream, capture, plan, ws, plan_bytes, ws_bytes;
     int device, t, n, h;
-    if (!PyArg_ParseTuple(args, "KiKKKKiii", &stream, &device, &plan, &plan_bytes, &ws, &ws_bytes, &t, &n, &h)) return nullptr;
-    OpEntry* e = find_op(reinterpret_cast<void*>(stream), device);
+    if (!PyArg_ParseTuple(args, "KiKKKKKiii", &stream, &device, &capture, &plan, &plan_bytes, &ws, &ws_bytes, &t, &n, &h)) return nullptr;
+    void* s = reinterpret_cast<void*>(stream);
+    for (size_t i = g_ops->size(); i-- > 0;) {
+        const OpEntry& o = (*g_ops)[i];
+        if (o.stream == s && o.device == device && o.capture != 0 && o.capture != capture) g_ops->erase(g_ops->begin() + i);
+    }
+    OpEntry* e = find_op(s, device, capture);
     if (!e) { g_ops->emplace_back(); e = &g_ops->back(); }
-    e->stream = reinterpret_cast<void*>(stream); e->device = device;
+    e->stream = s; e->device = device; e->capture = capture;
     e->plan = reinterpret_cast<void*>(plan); e->plan_bytes = plan_bytes;
     e->ws = reinterpret_cast<void*>(ws); e->ws_bytes = ws_bytes;
     e->cap_t = t; e->cap_n = n; e->cap_h = h; e->built = false;
@@ -320,17 +324,17 @@ bool read_op(PyObject* const* args, OpArgs& a) {
     return !PyErr_Occurred();
 }
 
-// bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) -> status; kSlow also while this stream's plan
-// and workspace are missing or too small
+// bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) -> status; kSlow also while the plan and workspace of
+// this stream (or of the capture it is in) are missing or too small
 PyObject* py_bgmv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     OpArgs a;
     if (nargs != 7 || !read_op(args, a)) return slow();
     void* stream = stream_of(*a.x);
-    OpEntry* e = find_op(stream, a.ids->get_device());
-    if (!e || a.t > e->cap_t || a.n > e->cap_n || a.h_in > e->cap_h) return slow();
     unsigned long long cap = 0;
     int rc = b200_lora_stream_capture_id(stream, &cap);
     if (rc) return PyLong_FromLong(rc);
+    OpEntry* e = find_op(stream, a.ids->get_device(), cap);
+    if (!e || a.t > e->cap_t || a.n > e->cap_n || a.h_in > e->cap_h) return slow();
     const void* ids_ptr = a.ids->data_ptr();
     const bool versioned = !a.ids->is_inference();                  // inference tensors have no version counter
     const uint32_t version = versioned ? a.ids->_version() : 0;
@@ -338,7 +342,7 @@ PyObject* py_bgmv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const float scale = (float)a.scale;
     c10::TensorImpl* impl = a.ids->unsafeGetTensorImpl();
     const bool same = e->built && versioned && e->ids._unsafe_get_target() == impl && e->ids_ptr == ids_ptr && e->version == version &&
-                      e->ids_type == ids_type && e->t == a.t && e->n == a.n && e->r == a.r && e->scale == scale && e->capture == cap;
+                      e->ids_type == ids_type && e->t == a.t && e->n == a.n && e->r == a.r && e->scale == scale;
     b200_lora_adapters ad;
     memset(&ad, 0, sizeof(ad));
     ad.n_adapters = (int32_t)a.n; ad.n_layers = (int32_t)a.l; ad.r_pool = (int32_t)a.r; ad.scale = scale;
@@ -351,12 +355,12 @@ PyObject* py_bgmv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         rc = b200_lora_plan_build(plan, pb, cap_t, ids_ptr, ids_type == (int)at::kLong, (int32_t)a.t, &ad, stream);
         Py_END_ALLOW_THREADS
         if (rc) return PyLong_FromLong(rc);
-        e = find_op(stream, a.ids->get_device());                    // another thread may have registered a stream
+        e = find_op(stream, a.ids->get_device(), cap);               // another thread may have registered a stream
         if (!e || e->plan != plan) return slow();
         e->built = true;
         e->ids = c10::weak_intrusive_ptr<c10::TensorImpl>(a.ids->getIntrusivePtr());
         e->ids_ptr = ids_ptr; e->version = version; e->ids_type = ids_type;
-        e->t = (int)a.t; e->n = (int)a.n; e->r = (int)a.r; e->scale = scale; e->capture = cap;
+        e->t = (int)a.t; e->n = (int)a.n; e->r = (int)a.r; e->scale = scale;
     }
     const b200_lora_proj pj{a.x->data_ptr(), a.y->data_ptr(), a.wa->data_ptr(), a.wb->data_ptr(), a.h_in, a.h_out, (int32_t)a.h_in, (int32_t)a.h_out};
     void *plan = e->plan, *ws = e->ws;
@@ -384,12 +388,29 @@ PyObject* py_bgmv_static(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return PyLong_FromLong(rc);
 }
 
+// stream_key(tensor) -> (current stream of the tensor's device, identifier of the capture it is in or 0)
+PyObject* py_stream_key(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 1 || !THPVariable_Check(args[0]) || !THPVariable_Unpack(args[0]).is_cuda()) {
+        PyErr_SetString(PyExc_ValueError, "a CUDA tensor expected");
+        return nullptr;
+    }
+    void* stream = stream_of(THPVariable_Unpack(args[0]));
+    unsigned long long cap = 0;
+    const int rc = b200_lora_stream_capture_id(stream, &cap);
+    if (rc) {
+        PyErr_Format(PyExc_RuntimeError, "stream capture status: %s", b200_lora_last_cuda_error());
+        return nullptr;
+    }
+    return Py_BuildValue("(KK)", reinterpret_cast<unsigned long long>(stream), cap);
+}
+
 PyMethodDef kMethods[] = {
     {"apply", (PyCFunction)(void*)guarded<py_apply>, METH_FASTCALL, nullptr},
     {"plan_build", (PyCFunction)(void*)guarded<py_plan_build>, METH_FASTCALL, nullptr},
     {"plan_segments", (PyCFunction)(void*)guarded<py_plan_segments>, METH_FASTCALL, nullptr},
     {"bgmv", (PyCFunction)(void*)guarded<py_bgmv>, METH_FASTCALL, nullptr},
     {"bgmv_static", (PyCFunction)(void*)guarded<py_bgmv_static>, METH_FASTCALL, nullptr},
+    {"stream_key", (PyCFunction)(void*)guarded<py_stream_key>, METH_FASTCALL, nullptr},
     {"bgmv_register", py_bgmv_register, METH_VARARGS, nullptr},
     {"bgmv_forget", py_bgmv_forget, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},

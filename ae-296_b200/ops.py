@@ -195,7 +195,7 @@ def apply(projs: Sequence[Tuple[torch.Tensor, torch.Tensor, AdapterPool]], plan:
 
 
 # ---- the reference's operator call ---------------------------------------------------------------
-_OP_STATE = {}                       # (device, stream) -> (LoraBatch, capacity: tokens, adapters, h_in)
+_OP_STATE = {}                       # (device, stream, capture) -> (LoraBatch, capacity: tokens, adapters, h_in)
 
 
 def invalidate_plan_cache() -> None:
@@ -205,24 +205,27 @@ def invalidate_plan_cache() -> None:
     _lib.host().bgmv_forget()
 
 
-def _op_state(dev, t: int, n: int, h_in: int) -> None:
+def _op_state(ids: torch.Tensor, t: int, n: int, h_in: int) -> None:
     """Makes the plan and workspace behind :func:`add_lora_bgmv` for the current stream large enough.
 
     The reference's decode loop calls the op 3 x n_layers times per step with the SAME index tensor
     (lightllm/models/lora_gpu.py:138,150,162 with ``select_inds[bsz-1]``).  The plan depends on
     the ids, N, r and the scale only, so it is kept while the very same tensor is passed again
-    unmodified (torch's version counter) and rebuilt otherwise.  A plan built outside a
-    CUDA-graph capture is never used inside one, nor one capture's plan in another: the capture's
-    identifier is part of the key, so every graph contains the build of the plan it applies (its
-    first call) and replays rebuild it from the index tensor's contents of the moment.  The key lives in
-    the native host path; the memory is held here."""
-    stream = _stream(dev)
-    _, old = _OP_STATE.get((dev.index, stream), (None, (0, 0, 0)))
+    unmodified (torch's version counter) and rebuilt otherwise.  Every CUDA-graph capture has a plan and
+    workspace of its own, allocated inside it (so that the graph's memory pool owns them), and contains the
+    build of the plan it applies (its first call): replays rebuild it from the index tensor's contents of the
+    moment and touch nothing that eager calls or other graphs use.  The key lives in the native host path;
+    the memory is held here, an ended capture's until the stream's next entry is made."""
+    dev = ids.device.index
+    stream, capture = _lib.host().stream_key(ids)
+    for key in [k for k in _OP_STATE if k[:2] == (dev, stream) and k[2] not in (0, capture)]:
+        del _OP_STATE[key]
+    _, old = _OP_STATE.get((dev, stream, capture), (None, (0, 0, 0)))
     dims = (max(t, old[0]), max(n, old[1]), max(h_in, old[2]))
-    batch = LoraBatch(*dims, 1, dev)
-    _OP_STATE[dev.index, stream] = (batch, dims)
-    _lib.host().bgmv_register(stream, dev.index, batch.plan.buf.data_ptr(), batch.plan.nbytes,
+    batch = LoraBatch(*dims, 1, ids.device)
+    _lib.host().bgmv_register(stream, dev, capture, batch.plan.buf.data_ptr(), batch.plan.nbytes,
                               batch.workspace.buf.data_ptr(), batch.workspace.nbytes, *dims)
+    _OP_STATE[dev, stream, capture] = (batch, dims)
 
 
 def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T_all: torch.Tensor,
@@ -257,7 +260,7 @@ def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T
         raise ValueError("fp16 or bf16 tensors of one dtype expected")
     if indicies.dtype not in (torch.int32, torch.int64):
         raise ValueError("indicies must be int32 or int64")
-    _op_state(indicies.device, t, n, h_in)
+    _op_state(indicies, t, n, h_in)
     rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
     if rc > 0:
         raise ValueError("add_lora_bgmv: unsupported arguments")
