@@ -20,6 +20,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -246,7 +247,10 @@ PyObject* py_plan_segments(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // Python side, which registers it here; what the plan was built from is kept here.  A capture has an entry of
 // its own, since every replay writes the plan again: an eager call must not find its plan replaced by a replay.
 // The index tensor is held weakly: its object stays comparable by address, its storage does not stay alive.
+// `mu` holds a call's enqueues together: another thread's plan must not come between a call's plan, its key and
+// its apply.  It is only taken without the GIL (a launch may wait for the GPU, and the GPU for a host callback).
 struct OpEntry {
+    std::mutex mu;
     void* stream = nullptr;
     int device = -1;
     unsigned long long capture = 0;
@@ -260,37 +264,65 @@ struct OpEntry {
     int ids_type = 0, t = 0, n = 0, r = 0;
     float scale = 0.f;
 };
-std::vector<OpEntry>* g_ops;       // guarded by the GIL; a process has a handful of streams
+using OpRef = std::shared_ptr<OpEntry>;
+std::vector<OpRef>* g_ops;         // guarded by the GIL; a process has a handful of streams
 
-OpEntry* find_op(void* stream, int device, unsigned long long capture) {
-    for (OpEntry& e : *g_ops)
-        if (e.stream == stream && e.device == device && e.capture == capture) return &e;
+OpRef find_op(void* stream, int device, unsigned long long capture) {
+    for (const OpRef& e : *g_ops)
+        if (e->stream == stream && e->device == device && e->capture == capture) return e;
     return nullptr;
 }
 
+struct NoGil {
+    PyThreadState* state;
+    NoGil() : state(PyEval_SaveThread()) {}
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // bgmv_register(stream, device, capture, plan_ptr, plan_bytes, ws_ptr, ws_bytes, cap_t, cap_n, cap_h)
 // A stream is in one capture at a time: entries of its earlier captures go.
-PyObject* py_bgmv_register(PyObject*, PyObject* args) {
+bool register_op(PyObject* args) {
     unsigned long long stream, capture, plan, ws, plan_bytes, ws_bytes;
     int device, t, n, h;
-    if (!PyArg_ParseTuple(args, "KiKKKKKiii", &stream, &device, &capture, &plan, &plan_bytes, &ws, &ws_bytes, &t, &n, &h)) return nullptr;
+    if (!PyArg_ParseTuple(args, "KiKKKKKiii", &stream, &device, &capture, &plan, &plan_bytes, &ws, &ws_bytes, &t, &n, &h)) return false;
     void* s = reinterpret_cast<void*>(stream);
     for (size_t i = g_ops->size(); i-- > 0;) {
-        const OpEntry& o = (*g_ops)[i];
+        const OpEntry& o = *(*g_ops)[i];
         if (o.stream == s && o.device == device && o.capture != 0 && o.capture != capture) g_ops->erase(g_ops->begin() + i);
     }
-    OpEntry* e = find_op(s, device, capture);
-    if (!e) { g_ops->emplace_back(); e = &g_ops->back(); }
-    e->stream = s; e->device = device; e->capture = capture;
+    OpRef e = find_op(s, device, capture);
+    if (!e) {
+        e = std::make_shared<OpEntry>();
+        e->stream = s; e->device = device; e->capture = capture;
+        g_ops->push_back(e);
+    }
+    NoGil nogil;
+    std::lock_guard<std::mutex> lock(e->mu);
     e->plan = reinterpret_cast<void*>(plan); e->plan_bytes = plan_bytes;
     e->ws = reinterpret_cast<void*>(ws); e->ws_bytes = ws_bytes;
     e->cap_t = t; e->cap_n = n; e->cap_h = h; e->built = false;
+    return true;
+}
+PyObject* py_bgmv_register(PyObject*, PyObject* args) {
+    try {
+        if (!register_op(args)) return nullptr;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
     Py_RETURN_NONE;
 }
 
 // bgmv_forget(): the plans must be rebuilt on their next use
-PyObject* py_bgmv_forget(PyObject*, PyObject*) {
-    for (OpEntry& e : *g_ops) e.built = false;
+PyObject* py_bgmv_forget(PyObject*, PyObject* const*, Py_ssize_t) {
+    const std::vector<OpRef> all(*g_ops);
+    {
+        NoGil nogil;
+        for (const OpRef& e : all) {
+            std::lock_guard<std::mutex> lock(e->mu);
+            e->built = false;
+        }
+    }
     Py_RETURN_NONE;
 }
 
@@ -333,43 +365,38 @@ PyObject* py_bgmv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     unsigned long long cap = 0;
     int rc = b200_lora_stream_capture_id(stream, &cap);
     if (rc) return PyLong_FromLong(rc);
-    OpEntry* e = find_op(stream, a.ids->get_device(), cap);
-    if (!e || a.t > e->cap_t || a.n > e->cap_n || a.h_in > e->cap_h) return slow();
-    const void* ids_ptr = a.ids->data_ptr();
+    const OpRef e = find_op(stream, a.ids->get_device(), cap);
+    if (!e) return slow();
     const bool versioned = !a.ids->is_inference();                  // inference tensors have no version counter
     const uint32_t version = versioned ? a.ids->_version() : 0;
     const int ids_type = (int)a.ids->scalar_type();
     const float scale = (float)a.scale;
-    c10::TensorImpl* impl = a.ids->unsafeGetTensorImpl();
-    const bool same = e->built && versioned && e->ids._unsafe_get_target() == impl && e->ids_ptr == ids_ptr && e->version == version &&
-                      e->ids_type == ids_type && e->t == a.t && e->n == a.n && e->r == a.r && e->scale == scale;
+    const void* ids_ptr = a.ids->data_ptr();
+    c10::weak_intrusive_ptr<c10::TensorImpl> ids(a.ids->getIntrusivePtr());
     b200_lora_adapters ad;
     memset(&ad, 0, sizeof(ad));
     ad.n_adapters = (int32_t)a.n; ad.n_layers = (int32_t)a.l; ad.r_pool = (int32_t)a.r; ad.scale = scale;
-    if (!same) {
-        e->built = false;
-        void* plan = e->plan;
-        const size_t pb = e->plan_bytes;
-        const int cap_t = e->cap_t;
-        Py_BEGIN_ALLOW_THREADS
-        rc = b200_lora_plan_build(plan, pb, cap_t, ids_ptr, ids_type == (int)at::kLong, (int32_t)a.t, &ad, stream);
-        Py_END_ALLOW_THREADS
-        if (rc) return PyLong_FromLong(rc);
-        e = find_op(stream, a.ids->get_device(), cap);               // another thread may have registered a stream
-        if (!e || e->plan != plan) return slow();
-        e->built = true;
-        e->ids = c10::weak_intrusive_ptr<c10::TensorImpl>(a.ids->getIntrusivePtr());
-        e->ids_ptr = ids_ptr; e->version = version; e->ids_type = ids_type;
-        e->t = (int)a.t; e->n = (int)a.n; e->r = (int)a.r; e->scale = scale;
-    }
     const b200_lora_proj pj{a.x->data_ptr(), a.y->data_ptr(), a.wa->data_ptr(), a.wb->data_ptr(), a.h_in, a.h_out, (int32_t)a.h_in, (int32_t)a.h_out};
-    void *plan = e->plan, *ws = e->ws;
-    const size_t wb = e->ws_bytes;
-    const int cap_t = e->cap_t;
-    Py_BEGIN_ALLOW_THREADS
-    rc = b200_lora_apply(&pj, 1, &ad, plan, cap_t, (int32_t)a.t, (int32_t)a.layer, a.io, a.io, B200_LORA_NO_TENSOR, ws, wb, stream);
-    Py_END_ALLOW_THREADS
-    return PyLong_FromLong(rc);
+    {
+        NoGil nogil;
+        std::lock_guard<std::mutex> lock(e->mu);
+        if (a.t > e->cap_t || a.n > e->cap_n || a.h_in > e->cap_h) rc = kSlow;
+        const bool same = e->built && versioned && e->ids._unsafe_get_target() == ids._unsafe_get_target() && e->ids_ptr == ids_ptr &&
+                          e->version == version && e->ids_type == ids_type && e->t == a.t && e->n == a.n && e->r == a.r && e->scale == scale;
+        if (rc == 0 && !same) {
+            e->built = false;
+            rc = b200_lora_plan_build(e->plan, e->plan_bytes, e->cap_t, ids_ptr, ids_type == (int)at::kLong, (int32_t)a.t, &ad, stream);
+            if (rc == 0) {
+                e->built = true;
+                std::swap(e->ids, ids);                             // the former one is released with the GIL held
+                e->ids_ptr = ids_ptr; e->version = version; e->ids_type = ids_type;
+                e->t = (int)a.t; e->n = (int)a.n; e->r = (int)a.r; e->scale = scale;
+            }
+        }
+        if (rc == 0)
+            rc = b200_lora_apply(&pj, 1, &ad, e->plan, e->cap_t, (int32_t)a.t, (int32_t)a.layer, a.io, a.io, B200_LORA_NO_TENSOR, e->ws, e->ws_bytes, stream);
+    }
+    return rc == kSlow ? slow() : PyLong_FromLong(rc);
 }
 
 // bgmv_static(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale) -> status
@@ -412,7 +439,7 @@ PyMethodDef kMethods[] = {
     {"bgmv_static", (PyCFunction)(void*)guarded<py_bgmv_static>, METH_FASTCALL, nullptr},
     {"stream_key", (PyCFunction)(void*)guarded<py_stream_key>, METH_FASTCALL, nullptr},
     {"bgmv_register", py_bgmv_register, METH_VARARGS, nullptr},
-    {"bgmv_forget", py_bgmv_forget, METH_NOARGS, nullptr},
+    {"bgmv_forget", (PyCFunction)(void*)guarded<py_bgmv_forget>, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
@@ -427,6 +454,6 @@ PyMODINIT_FUNC PyInit__b200host(void) {
         {&s_max_tokens, "max_tokens"}, {&s_n_tokens, "n_tokens"}};
     for (auto& e : names)
         if (!(*e.slot = PyUnicode_InternFromString(e.name))) return nullptr;
-    g_ops = new std::vector<OpEntry>();
+    g_ops = new std::vector<OpRef>();
     return PyModule_Create(&kModule);
 }

@@ -16,6 +16,7 @@ missing.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -196,6 +197,7 @@ def apply(projs: Sequence[Tuple[torch.Tensor, torch.Tensor, AdapterPool]], plan:
 
 # ---- the reference's operator call ---------------------------------------------------------------
 _OP_STATE = {}                       # (device, stream, capture) -> (LoraBatch, capacity: tokens, adapters, h_in)
+_OP_LOCK = threading.Lock()
 
 
 def invalidate_plan_cache() -> None:
@@ -218,14 +220,18 @@ def _op_state(ids: torch.Tensor, t: int, n: int, h_in: int) -> None:
     the memory is held here, an ended capture's until the stream's next entry is made."""
     dev = ids.device.index
     stream, capture = _lib.host().stream_key(ids)
-    for key in [k for k in _OP_STATE if k[:2] == (dev, stream) and k[2] not in (0, capture)]:
-        del _OP_STATE[key]
-    _, old = _OP_STATE.get((dev, stream, capture), (None, (0, 0, 0)))
-    dims = (max(t, old[0]), max(n, old[1]), max(h_in, old[2]))
-    batch = LoraBatch(*dims, 1, ids.device)
-    _lib.host().bgmv_register(stream, dev, capture, batch.plan.buf.data_ptr(), batch.plan.nbytes,
-                              batch.workspace.buf.data_ptr(), batch.workspace.nbytes, *dims)
-    _OP_STATE[dev, stream, capture] = (batch, dims)
+    with _OP_LOCK:
+        for key in [k for k in _OP_STATE if k[:2] == (dev, stream) and k[2] not in (0, capture)]:
+            del _OP_STATE[key]
+        _, old = _OP_STATE.get((dev, stream, capture), (None, (0, 0, 0)))
+        dims = (max(t, old[0]), max(n, old[1]), max(h_in, old[2]))
+        if dims == old:                  # another thread has made it meanwhile
+            return
+        batch = LoraBatch(*dims, 1, ids.device)
+        # registered before the old memory goes: no call can still be enqueueing with that then
+        _lib.host().bgmv_register(stream, dev, capture, batch.plan.buf.data_ptr(), batch.plan.nbytes,
+                                  batch.workspace.buf.data_ptr(), batch.workspace.nbytes, *dims)
+        _OP_STATE[dev, stream, capture] = (batch, dims)
 
 
 def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T_all: torch.Tensor,

@@ -1,5 +1,7 @@
 """Plans and workspaces that calls keep for the next one: graph captures, streams and threads must not see each
 other's."""
+import threading
+
 import pytest
 import torch
 
@@ -80,3 +82,34 @@ def test_operator_graphs_of_growing_batches_keep_their_memory():
     for _, y, want, _ in graphs:
         assert torch.equal(y, want)
     assert all(bool((o == 7).all()) for o in others)
+
+
+def test_operator_called_by_threads_on_one_stream():
+    """Threads that share a stream share its plan: no call may run with the ids of another thread's, also while
+    the batches grow."""
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    jobs = []
+    for k in range(4):
+        x, wa, wb, (ids, _) = _op_inputs(24 + 8 * k, 50 + k)
+        jobs.append((x, wa, wb, ids, _once(x, wa, wb, ids)))
+    torch.cuda.synchronize()
+    wrong, errors = [], []
+
+    def work(x, wa, wb, ids, want):
+        try:
+            with torch.cuda.stream(s):
+                ys = [torch.zeros_like(want) for _ in range(400)]
+                for y in ys:
+                    L.add_lora_bgmv(y, x, wa, wb, ids, 0, 1.0)
+                s.synchronize()
+                wrong.append(sum(not torch.equal(y, want) for y in ys))
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and wrong == [0] * len(jobs)
