@@ -7,7 +7,7 @@ lightllm/models/lora_gpu.py:16-163, so the layer-infer code
 unchanged.  Differences, all on purpose:
 
 * the decode op is this package's CUDA BGMV instead of ``punica.ops.add_lora_bgmv``, with one
-  plan per batch size (built once, not per call) and q/k/v of a layer computed in one fused pass;
+  plan per batch size and stream (built once per ``set_indices``, not per call) and q/k/v of a layer computed in one fused pass;
 * prefill uses the same kernels on request-aligned segments (slot ``b`` <-> request ``b``)
   instead of two ``torch.bmm`` calls and two transposed copies; ``prefill_mid_round``
   reproduces that op's fp16 rounding of the ``[B, L, r]`` intermediate;
@@ -26,6 +26,14 @@ import numpy as np
 from . import _lib
 from .ops import LoraBatch, _adapters_struct, apply
 from .pool import AdapterPool
+
+
+class _Kept:
+    """A plan + workspace that calls of one kind keep, and what the plan was built from."""
+
+    def __init__(self, batch: LoraBatch):
+        self.batch = batch
+        self.built = None
 
 
 class Lora_GPU:
@@ -70,19 +78,31 @@ class Lora_GPU:
                                 (self.v_down_prefill, self.v_up_prefill))]
         self._ad_decode = _adapters_struct(self.batch_size, self.n_layers, self.lora_rank, scale=1.0)
         self._ad_prefill = _adapters_struct(self.max_prefill_batch_size, self.n_layers, self.lora_rank, scale=1.0)
-        # one plan + workspace per decode batch size in use (built by the first call or by
-        # set_indices), one for prefill that grows to the largest batch seen
-        self._decode_batch = {}
-        self._decode_stale = set()       # batch sizes whose plan has to be rebuilt (set_indices)
-        self._prefill_batch = None
-        self._prefill_shape = None
+        # Plan + workspace per (decode batch size, or None for prefill; stream; graph capture or 0), so that a
+        # step on another stream, and every replay of a graph, which builds its plan again, leaves this one's alone.
+        self._kept = {}
+        self._stream_key = _lib.host().stream_key
+        self._indices_version = {}       # decode batch size -> how often set_indices has set it
         self._fused = None               # (x identity, layer, prefill) -> the k and v deltas computed with q
 
     def set_indices(self, indices: torch.Tensor) -> None:
-        """Adapter slot of each decode token for batches of ``len(indices)`` tokens."""
+        """Adapter slot of each decode token for batches of ``len(indices)`` tokens.  A captured graph goes on
+        with the index tensor that it was captured with (its contents at each replay), which the caller keeps."""
         bsz = indices.numel()
         self.select_inds[bsz - 1] = indices.to(device=f"cuda:{self.device}")
-        self._decode_stale.add(bsz)
+        self._indices_version[bsz] = self._indices_version.get(bsz, 0) + 1
+
+    def _keep(self, x, kind, rows, n_adapters) -> _Kept:
+        """What is kept for calls of ``kind`` on the stream (and in the capture) that ``x`` is used on, with room
+        for ``rows``.  A capture's is allocated inside it, so its memory belongs to the graph's pool; the
+        reference here goes when the stream, which is in one capture at a time, makes its next."""
+        where = self._stream_key(x)
+        kept = self._kept.get((kind, where))
+        if kept is None or kept.batch.plan.max_tokens < rows:
+            for key in [k for k in self._kept if k[1][0] == where[0] and k[1][1] not in (0, where[1])]:
+                del self._kept[key]
+            kept = self._kept[kind, where] = _Kept(LoraBatch(rows, n_adapters, self.in_size, 3, x.device))
+        return kept
 
     # ---- the three calls the layer code makes ------------------------------------------
     # The layer code asks for q, k and v of one layer in that order with the same input
@@ -118,33 +138,30 @@ class Lora_GPU:
     def _decode(self, x, layer_id, projs):
         """x ``[bsz, H]``; token ``t`` uses slot ``select_inds[bsz-1][t]`` (lora_gpu.py:137-138)."""
         bsz = x.shape[0]
-        batch = self._decode_batch.get(bsz)
-        if batch is None:
-            batch = self._decode_batch[bsz] = LoraBatch(bsz, self.batch_size, self.in_size, 3, x.device)
-            self._decode_stale.add(bsz)
-        if bsz in self._decode_stale:
+        kept = self._keep(x, bsz, bsz, self.batch_size)
+        batch = kept.batch
+        version = self._indices_version.get(bsz, 0)
+        if kept.built != version:
             batch.plan.build(self.select_inds[bsz - 1], self._ad_decode)
-            self._decode_stale.discard(bsz)
+            kept.built = version
         y = torch.empty(3, bsz, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
         apply([(x, y[i], self._decode_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace,
               _lib.NO_TENSOR | _lib.OVERWRITE, self._ad_decode)
-        return {i: y[i] for i in projs}
+        return y                         # only those of `projs` hold anything
 
     def _prefill(self, x, layer_id, projs):
         """x ``[B, L, H]``: request ``b`` uses prefill slot ``b`` (lora_gpu.py:125-128).  One plan +
-        workspace serves every shape: it grows to the largest batch seen and the segment table is
+        workspace (per stream) serves every shape: it grows to the largest batch seen and the segment table is
         rebuilt (one small kernel) when ``(B, L)`` changes, so nothing accumulates per shape."""
         bsz, seqlen, hidden = x.shape
         rows = bsz * seqlen
-        if self._prefill_batch is None or rows > self._prefill_batch.plan.max_tokens:
-            self._prefill_batch = LoraBatch(rows, self.max_prefill_batch_size, self.in_size, 3, x.device)
-            self._prefill_shape = None
-        batch = self._prefill_batch
-        if self._prefill_shape != (bsz, seqlen):
+        kept = self._keep(x, None, rows, self.max_prefill_batch_size)
+        batch = kept.batch
+        if kept.built != (bsz, seqlen):
             starts = torch.arange(0, (bsz + 1) * seqlen, seqlen, dtype=torch.int32, device=x.device)
             slots = torch.arange(bsz, dtype=torch.int32, device=x.device)
             batch.plan.from_segments(starts, slots, rows, self._ad_prefill)
-            self._prefill_shape = (bsz, seqlen)
+            kept.built = (bsz, seqlen)
         y = torch.empty(3, rows, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
         flags = _lib.OVERWRITE | (_lib.MID_ROUND if self.prefill_mid_round else 0)
         x2 = x.reshape(rows, hidden)

@@ -113,3 +113,113 @@ def test_operator_called_by_threads_on_one_stream():
     for t in threads:
         t.join()
     assert not errors and wrong == [0] * len(jobs)
+
+
+# ---- the layer object ----------------------------------------------------------------------------
+def _layer_object(T=24):
+    torch.manual_seed(3)
+    obj = L.Lora_GPU({"n_layers": 2, "batch_size": 32, "lora_rank": 16, "hidden_dim": H, "tp_degree": 1,
+                      "max_prefill_batch_size": 6})
+    x = torch.randn(T, H, device="cuda").half()
+    ids = [torch.randint(0, 32, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(k)) for k in range(2)]
+
+    def want(i):
+        y = torch.zeros_like(x)
+        ws = torch.empty(L.add_lora_bgmv_workspace_bytes(T, 32, H), dtype=torch.uint8, device="cuda")
+        L.add_lora_bgmv_once(y, x, obj.q_down, obj.q_up, ids[i], 1, 1.0, ws)
+        return y.float()
+
+    def same(got, i):                     # the fused call cuts the split-K sums elsewhere: one ulp
+        w = want(i)
+        torch.cuda.synchronize()
+        return bool(((got.float() - w).abs() <= 2.0 ** -10 * w.abs() + 2.0 ** -24).all())
+
+    return obj, x, ids, same
+
+
+def test_layer_object_eager_steps_after_replays():
+    """A graph captured with one set of indices, eager steps with another before and after its replay."""
+    obj, x, (a, b), same = _layer_object()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    out = {}
+    with torch.cuda.stream(s):
+        obj.set_indices(a)
+        obj.invoke_one_layer_q(x, 1)                       # warm-up
+        obj.set_indices(a)
+        g = _capture(s, lambda: out.update(g=obj.invoke_one_layer_q(x, 1)))
+        obj.set_indices(b)
+        before = obj.invoke_one_layer_q(x, 1)
+        g.replay()
+        after = obj.invoke_one_layer_q(x, 1)
+    torch.cuda.synchronize()
+    assert same(before, 1) and same(out["g"], 0) and same(after, 1)
+
+
+def test_layer_object_eager_step_before_the_first_replay():
+    """A plan that was only captured has not been built: the eager step makes its own."""
+    obj, x, (a, b), same = _layer_object()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        obj.set_indices(a)
+        obj.invoke_one_layer_q(x, 1)
+        obj.set_indices(b)
+        _capture(s, lambda: obj.invoke_one_layer_q(x, 1))
+        eager = obj.invoke_one_layer_q(x, 1)
+    torch.cuda.synchronize()
+    assert same(eager, 1)
+
+
+def test_layer_object_graph_keeps_its_indices():
+    """set_indices and an eager step leave a captured graph with the indices of its capture."""
+    obj, x, (a, b), same = _layer_object()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    out = {}
+    with torch.cuda.stream(s):
+        obj.set_indices(a)
+        obj.invoke_one_layer_q(x, 1)                       # the plan exists: the capture must build it again
+        g = _capture(s, lambda: out.update(g=obj.invoke_one_layer_q(x, 1)))
+        obj.set_indices(b)
+        obj.invoke_one_layer_q(x, 1)
+        g.replay()
+    torch.cuda.synchronize()
+    assert same(out["g"], 0)
+
+
+def test_layer_object_on_two_streams():
+    """Steps with different indices in flight on two streams have plans and workspaces of their own."""
+    obj, x, (a, b), same = _layer_object()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    got = [[], []]
+    for _ in range(20):
+        for i, ids in enumerate((a, b)):
+            with torch.cuda.stream(streams[i]):
+                obj.set_indices(ids)
+                got[i] += [obj.invoke_one_layer_q(x, 1) for _ in range(3)]
+    torch.cuda.synchronize()
+    batches = {id(k.batch) for k in obj._kept.values()}
+    assert len(batches) == 2
+    assert all(same(y, i) for i in range(2) for y in got[i])
+
+
+def test_layer_object_prefill_shape_only_captured():
+    """As above for prefill: a shape whose segment table was only captured is built by the eager call."""
+    obj, _, _, _ = _layer_object()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    xs = [torch.randn(*shape, H, device="cuda").half() for shape in ((2, 60), (3, 40))]
+    with torch.cuda.stream(s):
+        obj.invoke_one_layer_q(xs[0], 1, prefill=True)
+        _capture(s, lambda: obj.invoke_one_layer_q(xs[1], 1, prefill=True))
+        got = obj.invoke_one_layer_q(xs[1], 1, prefill=True)
+    torch.cuda.synchronize()
+    for i in range(3):
+        v = (xs[1][i].float() @ obj.q_down_prefill[i, 1].float().t()).half().float()
+        want = v @ obj.q_up_prefill[i, 1].float().t()
+        rms = float(want.pow(2).mean().sqrt())
+        # one rounding of the result, and of an intermediate that may fall on the other side of a tie
+        assert float((got[i].float() - want).abs().max()) <= 2e-3 * rms + float(want.abs().max()) * 2 ** -10
