@@ -20,6 +20,8 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <string.h>
+
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -75,7 +77,8 @@ bool dtype_code(at::ScalarType t, int& code) {
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
 // The adapter table of a pool object, or of a ctypes structure of the same layout.  The ranks are read from
-// the pool's host copy on every call: a pool manager may change a slot's rank between calls.
+// the pool's host copy on every call: a pool manager may change a slot's rank between calls.  Host tables of other
+// types than int32 ranks and int64 prefixes are the Python code's to read.
 bool read_adapters(PyObject* obj, b200_lora_adapters& ad) {
     if (PyObject_CheckBuffer(obj)) {
         Py_buffer b;
@@ -100,8 +103,8 @@ bool read_adapters(PyObject* obj, b200_lora_adapters& ad) {
     Ref rh(PyObject_GetAttr(obj, s_ranks_host)), ch(PyObject_GetAttr(obj, s_cum_host));
     if (!rh || !ch || !PyObject_CheckBuffer(rh.o) || !PyObject_CheckBuffer(ch.o)) return false;
     Py_buffer b;
-    if (PyObject_GetBuffer(rh.o, &b, PyBUF_SIMPLE) != 0) return false;
-    bool ok = b.itemsize == 4 && b.len == 4 * n;
+    if (PyObject_GetBuffer(rh.o, &b, PyBUF_ND | PyBUF_FORMAT) != 0) return false;
+    bool ok = b.format && b.itemsize == 4 && !strcmp(b.format, "i") && b.len == 4 * n;
     if (ok) {
         const int32_t* h = static_cast<const int32_t*>(b.buf);
         bool pow2 = true;
@@ -110,8 +113,8 @@ bool read_adapters(PyObject* obj, b200_lora_adapters& ad) {
         ad.ranks_pow2 = pow2 && (packed || r == 8 || r == 16 || r == 32 || r == 64);
     }
     PyBuffer_Release(&b);
-    if (!ok || PyObject_GetBuffer(ch.o, &b, PyBUF_SIMPLE) != 0) return false;
-    ok = b.itemsize == 8 && b.len >= 8;
+    if (!ok || PyObject_GetBuffer(ch.o, &b, PyBUF_ND | PyBUF_FORMAT) != 0) return false;
+    ok = b.format && b.itemsize == 8 && (!strcmp(b.format, "l") || !strcmp(b.format, "q")) && b.len >= 8;
     if (ok) ad.total_rank = static_cast<const int64_t*>(b.buf)[b.len / 8 - 1];
     PyBuffer_Release(&b);
     return ok;

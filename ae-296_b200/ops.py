@@ -61,6 +61,10 @@ def adapters_of(pool: AdapterPool) -> Adapters:
                             pool.cum_ranks, pool.packed, 1.0, pow2, int(pool.cum_host[-1]))
 
 
+def _table(adapters) -> Adapters:
+    return adapters if isinstance(adapters, Adapters) else adapters_of(adapters)
+
+
 class LoraPlan:
     """Device-resident segment table of one batch (see ``b200_lora_plan_build``)."""
 
@@ -80,7 +84,12 @@ class LoraPlan:
         _require_cuda(ids)
         if ids.dtype not in (torch.int32, torch.int64) or not ids.is_contiguous():
             raise ValueError("ids must be a contiguous int32/int64 tensor")
-        check(_lib.host().plan_build(self, ids, adapters), "plan_build")
+        rc = _lib.host().plan_build(self, ids, adapters)
+        if rc > 0:
+            rc = _lib.host().plan_build(self, ids, _table(adapters))
+        if rc > 0:
+            raise ValueError("plan_build: unsupported arguments")
+        check(rc, "plan_build")
         return self
 
     def from_segments(self, seg_starts: torch.Tensor, seg_adapter: torch.Tensor, n_tokens: int,
@@ -92,6 +101,8 @@ class LoraPlan:
             raise ValueError("segment tables must be int32")
         self._keep = (seg_starts, seg_adapter)
         rc = _lib.host().plan_segments(self, seg_starts, seg_adapter, int(n_tokens), adapters)
+        if rc > 0:
+            rc = _lib.host().plan_segments(self, seg_starts, seg_adapter, int(n_tokens), _table(adapters))
         if rc > 0:
             raise ValueError("segment tables are contiguous: one start per segment, and optionally the end of the last")
         check(rc, "plan_from_segments")
@@ -267,7 +278,7 @@ def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T
     if indicies.dtype not in (torch.int32, torch.int64):
         raise ValueError("indicies must be int32 or int64")
     _op_state(indicies, t, n, h_in)
-    rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
+    rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, int(layer_idx), float(scale))
     if rc > 0:
         raise ValueError("add_lora_bgmv: unsupported arguments")
     check(rc, "add_lora_bgmv")
@@ -323,7 +334,10 @@ def add_lora_bgmv_static(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tenso
         raise ValueError("fp16 or bf16 tensors of one dtype expected")
     if indicies.dtype not in (torch.int32, torch.int64):
         raise ValueError("indicies must be int32 or int64")
-    raise ValueError("add_lora_bgmv_static: unsupported arguments")
+    rc = _lib.host().bgmv_static(y, x, wa_T_all, wb_T_all, indicies, int(layer_idx), float(scale))
+    if rc > 0:
+        raise ValueError("add_lora_bgmv_static: unsupported arguments")
+    check(rc, "add_lora_bgmv_static")
 
 
 def add_lora_bgmv_static_status(device=None) -> None:

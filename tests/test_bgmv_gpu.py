@@ -214,6 +214,30 @@ def test_errors_are_raised_not_swallowed():
         L.add_lora_bgmv(y.cpu(), c.x.cpu(), c.pool.wa.cpu(), c.pool.wb.cpu(), c.ids_dev.cpu(), 0, 1.0)
 
 
+@pytest.mark.parametrize("host_type", [np.int64, np.float32])
+def test_pools_whose_host_ranks_have_another_type(host_type):
+    c = Case(20, 5, 256, 384, [8, 16, 64], "fp16", seed=4, n_layers=1)
+    want = c.run(0)
+    c.pool.ranks_host = c.pool.ranks_host.astype(host_type)
+    assert torch.equal(c.run(0), want)
+    order = np.argsort(c.ids, kind="stable")
+    starts = torch.from_numpy(np.searchsorted(c.ids[order], np.arange(6)).astype(np.int32)).cuda()
+    used = torch.unique_consecutive(starts)
+    owner = c.ids_dev[torch.from_numpy(order).cuda()][used[:-1].long()]
+    y = torch.zeros_like(want)
+    L.LoraBatch(20, 5, 256, 1).set_segments(used, owner, 20, c.pool).apply([(c.x[torch.from_numpy(order).cuda()], y, c.pool)], 0)
+    assert torch.equal(y, want[torch.from_numpy(order).cuda()])
+
+
+def test_numbers_of_other_types_as_layer_and_scale():
+    c = Case(7, 4, 128, 256, 16, "fp16", dense=True, seed=6)
+    for op in (L.add_lora_bgmv, L.add_lora_bgmv_static):
+        ys = [torch.zeros(7, 256, dtype=torch.float16, device="cuda") for _ in range(3)]
+        for y, layer, scale in zip(ys, (1, 1.0, np.float32(1)), (0.5, np.float32(0.5), "0.5")):
+            op(y, c.x, c.pool.wa, c.pool.wb, c.ids_dev, layer, scale)
+        assert ys[0].any() and torch.equal(ys[1], ys[0]) and torch.equal(ys[2], ys[0])
+
+
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_delta_then_add_mode(dtype):
     """The reference adds the 16-bit delta to the projection in 16-bit arithmetic (q += q_lora)."""
