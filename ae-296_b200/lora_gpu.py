@@ -31,8 +31,8 @@ from .pool import AdapterPool
 class _Kept:
     """A plan + workspace that calls of one kind keep, and what the plan was built from."""
 
-    def __init__(self, batch: LoraBatch):
-        self.batch = batch
+    def __init__(self, batch: LoraBatch, rows: int):
+        self.batch, self.rows = batch, rows
         self.built = None
 
 
@@ -98,10 +98,10 @@ class Lora_GPU:
         reference here goes when the stream, which is in one capture at a time, makes its next."""
         where = self._stream_key(x)
         kept = self._kept.get((kind, where))
-        if kept is None or kept.batch.plan.max_tokens < rows:
+        if kept is None or kept.rows < rows:
             for key in [k for k in self._kept if k[1][0] == where[0] and k[1][1] not in (0, where[1])]:
                 del self._kept[key]
-            kept = self._kept[kind, where] = _Kept(LoraBatch(rows, n_adapters, self.in_size, 3, x.device))
+            kept = self._kept[kind, where] = _Kept(LoraBatch(rows, n_adapters, self.in_size, 3, x.device), rows)
         return kept
 
     # ---- the three calls the layer code makes ------------------------------------------
@@ -144,7 +144,7 @@ class Lora_GPU:
         if kept.built != version:
             batch.plan.build(self.select_inds[bsz - 1], self._ad_decode)
             kept.built = version
-        y = torch.empty(3, bsz, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
+        y = x.new_empty((3, bsz, self.output_size)).unbind(0)
         apply([(x, y[i], self._decode_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace,
               _lib.NO_TENSOR | _lib.OVERWRITE, self._ad_decode)
         return y                         # only those of `projs` hold anything
@@ -162,7 +162,7 @@ class Lora_GPU:
             slots = torch.arange(bsz, dtype=torch.int32, device=x.device)
             batch.plan.from_segments(starts, slots, rows, self._ad_prefill)
             kept.built = (bsz, seqlen)
-        y = torch.empty(3, rows, self.output_size, device=x.device, dtype=x.dtype).unbind(0)
+        y = x.new_empty((3, rows, self.output_size)).unbind(0)
         flags = _lib.OVERWRITE | (_lib.MID_ROUND if self.prefill_mid_round else 0)
         x2 = x.reshape(rows, hidden)
         apply([(x2, y[i], self._prefill_pools[i]) for i in projs], batch.plan, layer_id, batch.workspace, flags,
