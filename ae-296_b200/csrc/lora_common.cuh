@@ -28,14 +28,15 @@ struct PlanHeader {
     int n_tokens;
     int n_segs;
     int n_units;      // sum over short segments of r_pad/8
-    int error;        // 0 ok, 1 adapter id out of range, 2 bad segment table, 3 rank promise broken
+    int error;        // 0 ok, 1 adapter id out of range, 2 bad segment table, 3 rank promise broken or above R
     int n_tiles;      // 128-row tiles of tall segments
     int cap;
     int n_adapters;
     int identity;     // 1: perm is the identity (rows pre-grouped)
     int n_units_short;  // units of short segments; they come first in unit_tab
     int n_wsegs;        // work segments
-    int pad[6];
+    int max_rank;       // largest rank of a segment
+    int pad[5];
 };
 static_assert(sizeof(PlanHeader) == 64, "plan header is 16 words");
 
@@ -194,15 +195,16 @@ __device__ __forceinline__ long long block_row0(const ApplyParams& p, const Unit
 __device__ __forceinline__ int b_pitch(const ApplyParams& p, int r) { return p.packed ? r : p.r_pool; }
 
 // Values of the workspace's sticky error word: 1..15 name the bounded wait that expired, this one
-// says that an apply call was given a plan built for another capacity or another number of rows.
+// says that an apply call was given a plan built for another capacity, another number of rows or wider adapters.
 constexpr unsigned kErrPlanMismatch = 64u;
 
 // May this apply walk the plan?  A plan whose build failed applies nothing (its own error word
 // tells why); a plan built for other sizes would index x and y out of range, so it applies
-// nothing either and the workspace's error word records it.
+// nothing either and the workspace's error word records it.  So with ranks above a dense pool's R: the
+// slots have no such rows, and the padded kernels no tensor map for such a class.
 __device__ __forceinline__ bool plan_usable(const PlanHeader& hdr, const ApplyParams& p, unsigned* err) {
     if (hdr.error) return false;
-    if (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens) {
+    if (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens || (!p.packed && hdr.max_rank > p.r_pool)) {
         if (threadIdx.x == 0) atomicMax(err, kErrPlanMismatch);
         return false;
     }

@@ -236,13 +236,16 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     const int kInf = 0x7fffffff;
     // segments: rank (checked against the promise made to the fast kernels), start marks
     for (int i = tid; i < T; i += NT) t0[i] = -1;
+    if (tid == 0) smem[44] = 0;                         // largest rank
     __syncthreads();
     for (int s = tid; s < S; s += NT) {
         const int a = sc.seg_adapter[s];
         int r = ranks ? ranks[a] : r_pool;
         if (ad.ranks_pow2 && !((r == 8 || r == 16 || r == 32 || r == 64) && (cum_ranks || r == r_pool)))
             pv.hdr->error = 3;                          // the fast kernels were promised these ranks
+        if (!cum_ranks && r > r_pool) pv.hdr->error = 3;    // a dense slot has R rows
         r = min(max(r, 1), kMaxRank);
+        atomicMax(&smem[44], r);
         pv.seg_rank[s] = r;
         pv.seg_flags[s] = 0;
         sc.seg_rank[s] = r;
@@ -365,6 +368,7 @@ __device__ void build_units(PlanView pv, const Scratch& sc, const PlanAdapters a
     }
     if (tid == 0) {
         pv.hdr->n_wsegs = tot_ws;
+        pv.hdr->max_rank = smem[44];
         pv.hdr->n_units = tot_short + tot_tall;
         pv.hdr->n_units_short = tot_short;
         pv.hdr->n_tiles = tot_tiles;

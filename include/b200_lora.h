@@ -77,7 +77,8 @@ typedef struct b200_lora_adapters {
     const int64_t* cum_ranks;  /* device [N+1] exclusive prefix of ranks; required when packed */
     int32_t n_adapters;        /* N */
     int32_t n_layers;          /* L */
-    int32_t r_pool;            /* R of the dense layout; upper bound of every rank */
+    int32_t r_pool;            /* R of the dense layout; upper bound of every rank.  A dense table with a larger one
+                                   yields B200_LORA_ERR_RANK from b200_lora_plan_read and a plan that applies nothing */
     int32_t packed;            /* 0 dense, 1 packed */
     float   scale;
     int32_t ranks_pow2;        /* caller's promise that every rank is 8, 16, 32 or 64 (and equals r_pool

@@ -227,3 +227,18 @@ def test_plan_of_another_batch_size_is_refused_on_the_device(shape):
     _lib.check(_lib.lib().b200_lora_workspace_init(batch.workspace.buf.data_ptr(), 64, torch.cuda.current_stream().cuda_stream))
     got = c.run(0, batch=batch)
     assert rel_err(got.double().cpu().numpy(), c.oracle_delta(0)) <= TOL + 2.0 ** -9
+
+
+@pytest.mark.parametrize("ranks", [16, [16, 3]])
+def test_plan_of_wider_adapters_is_refused_on_the_device(ranks):
+    """A plan that holds ranks above the applied dense pool's R: no slot has such rows."""
+    wide = Case(120, 6, 512, 512, 64, "fp16", dense=True, seed=8)
+    narrow = Case(120, 6, 512, 512, np.resize(np.array(ranks, np.int32), 6), "fp16", dense=True, seed=9)
+    batch = L.LoraBatch(120, 6, 512, 1).set_ids(wide.ids_dev, wide.pool)
+    y = torch.zeros(120, 512, dtype=torch.float16, device="cuda")
+    batch.apply([(narrow.x, y, narrow.pool)], 0)
+    torch.cuda.synchronize()
+    assert not y.any()
+    with pytest.raises(L.LoraError) as e:
+        batch.workspace.check()
+    assert e.value.code == -2

@@ -43,3 +43,26 @@ def test_plan_from_segments_round_trip_and_validation():
     with pytest.raises(L.LoraError) as e:
         plan.read()
     assert e.value.code == -10
+
+
+def test_dense_ranks_above_the_pools_are_refused():
+    """A slot of a dense pool has R rows: a table that says more (a stale one, or another pool's) makes a plan that
+    applies nothing.  Looked at through the plan alone."""
+    ids = torch.tensor([0, 1, 2, 1], dtype=torch.int32, device="cuda")
+    starts = torch.tensor([0, 1, 4], dtype=torch.int32, device="cuda")
+    plan = L.LoraPlan(4, 3)
+    for r_pool, ranks, code in [(16, [8, 24, 16], -5), (16, [16, 16, 3], 0), (24, [24, 12, 25], -5), (64, [64, 64, 64], 0),
+                                (16, [16, 64, 16], -5)]:
+        table = torch.tensor(ranks, dtype=torch.int32, device="cuda")
+        ad = _adapters_struct(3, 1, r_pool, ranks=table)
+        builds = [lambda: plan.build(ids, ad)]
+        if max(ranks[:2]) > r_pool or code == 0:           # the segment form uses adapters 0 and 1
+            builds.append(lambda: plan.from_segments(starts, ids[:2].contiguous(), 4, ad))
+        for build in builds:
+            build()
+            if code == 0:
+                plan.read()
+                continue
+            with pytest.raises(L.LoraError) as e:
+                plan.read()
+            assert e.value.code == code
