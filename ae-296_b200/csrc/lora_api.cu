@@ -169,7 +169,7 @@ bool fast_ranks(const b200_lora_adapters* ad) {
 //   h 2048, r 64 (2 CTAs an SM):  1 item 6.1 / 4.7   24 items 9.1 / 6.8   32 items 9.9 / 8.3   36 items 10.2 / 11.7
 // bgmv_cluster_limit() is 48 in the first row and falls with the CTAs that fit an SM.
 bool cluster_route(const ApplyParams& p, const b200_lora_adapters* ad, int io_dtype) {
-    if ((long long)p.n_tokens * p.n_proj > 1024) return false;       // far beyond any limit
+    if (p.n_tokens > kClusterTokens) return false;                   // beyond any limit, and what the plan has room for
     const int other = B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND | B200_LORA_DELTA_THEN_ADD;
     if (!(p.flags & B200_LORA_NO_TENSOR) || (p.flags & other) || !fast_ranks(ad) || !bgmv_cluster_fits(p)) return false;
     // a cluster writes its y rows while others still read x: not when the two share memory

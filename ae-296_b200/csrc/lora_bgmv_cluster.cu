@@ -332,7 +332,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     const Layout l = layout_of(p.r_cap, p.kcols, p.jcols);
     PlanView pv = plan_view(p.plan, p.cap, p.n_adapters);
     unsigned* err = &reinterpret_cast<WorkspaceCtl*>(p.workspace)->error;
-    // header and segment record in one round trip (the record of a segment the plan does not have is not used)
+    // header and segment record in one round trip (the record of a segment the plan does not have is not used; it is
+    // inside every plan, seg < kClusterTokens)
     UnitRec u;
     PlanHeader hdr;
     bool heads = true;

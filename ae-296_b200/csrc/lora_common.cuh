@@ -57,6 +57,9 @@ static_assert(sizeof(UnitRec) == 64, "unit record is 16 words");
 
 struct PlanView {
     PlanHeader* hdr;
+    int* seg_tab;       // [max(cap, 64)][16]  one unit record per work segment, in the order of the unit list.  The cluster
+                        // kernel reads it together with the header, before it knows that the plan was built for
+                        // the capacity it was told: so it lies at a place, and has room, that no capacity changes.
     int* perm;          // [cap]       sorted position -> token row
     int* seg_start;     // [cap + 1]   sorted position of each segment's first token
     int* seg_adapter;   // [cap]
@@ -67,15 +70,18 @@ struct PlanView {
     int* ws_rank;       // [cap]
     int* ws_unit0;      // [cap]       first unit record of the work segment
     int* unit_tab;      // [16 * cap][16]  one record per weight unit (see UnitRec)
-    int* seg_tab;       // [cap][16]   one unit record per work segment, in the order of the unit list
     int* tile_tab;      // [cap]       two words per tile of a tall run: first sorted position, (seg << 8) | (rows - 1)
     int* hist;          // [n_adapters + 1]
 };
 
+// tokens of the longest apply that may go to the cluster kernel
+constexpr int kClusterTokens = 64;
+__host__ __device__ inline size_t seg_tab_words(int cap) { return 16 * (size_t)(cap > kClusterTokens ? cap : kClusterTokens); }
+
 __host__ __device__ inline size_t plan_words(int cap, int n_adapters) {
-    // header + perm + seg_start + 3 seg arrays + units + tiles + hist, each padded to 4 words
+    // header + segment records + perm + seg_start + 3 seg arrays + units + tiles + hist, each padded to 4 words
     auto pad4 = [](size_t w) { return (w + 3) & ~size_t(3); };
-    return 16 + pad4(cap) + 2 * pad4(cap + 1) + 6 * pad4(cap) + 16 * kMaxSub * (size_t)cap + 16 * (size_t)cap + pad4(cap) +
+    return 16 + pad4(cap) + 2 * pad4(cap + 1) + 6 * pad4(cap) + 16 * kMaxSub * (size_t)cap + seg_tab_words(cap) + pad4(cap) +
            pad4((size_t)n_adapters + 1);
 }
 
@@ -84,6 +90,7 @@ __host__ __device__ inline PlanView plan_view(void* base, int cap, int n_adapter
     int* w = reinterpret_cast<int*>(base);
     PlanView v;
     v.hdr = reinterpret_cast<PlanHeader*>(w);      w += 16;
+    v.seg_tab = w;                                 w += seg_tab_words(cap);
     v.perm = w;                                    w += pad4(cap);
     v.seg_start = w;                               w += pad4(cap + 1);
     v.seg_adapter = w;                             w += pad4(cap);
@@ -94,7 +101,6 @@ __host__ __device__ inline PlanView plan_view(void* base, int cap, int n_adapter
     v.ws_rank = w;                                 w += pad4(cap);
     v.ws_unit0 = w;                                w += pad4(cap);
     v.unit_tab = w;                                w += 16 * kMaxSub * (size_t)cap;
-    v.seg_tab = w;                                 w += 16 * (size_t)cap;
     v.tile_tab = w;                                w += pad4(cap);
     v.hist = w;
     (void)n_adapters;

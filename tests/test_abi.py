@@ -29,6 +29,8 @@ def test_sizes_and_identification(lib):
     assert lib.b200_lora_arch() == 100
     assert lib.b200_lora_plan_bytes(256, 128) > 256 * 4 * 16
     assert lib.b200_lora_plan_bytes(0, 4) == 0
+    # an apply of up to 64 tokens reads a record per token behind the header before it can know the plan's capacity
+    assert all(lib.b200_lora_plan_bytes(cap, 1) >= 64 + 64 * 64 for cap in (1, 2, 40, 64))
     assert lib.b200_lora_workspace_bytes(256, 3, 4096) > 3 * 256 * 64 * 4
     assert lib.b200_lora_workspace_bytes(256, 5, 4096) == 0          # more than 4 projections
     off, size = C.c_size_t(0), C.c_size_t(0)

@@ -242,3 +242,18 @@ def test_plan_of_wider_adapters_is_refused_on_the_device(ranks):
     with pytest.raises(L.LoraError) as e:
         batch.workspace.check()
     assert e.value.code == -2
+
+
+def test_plan_of_another_capacity_is_refused_on_the_device():
+    """A caller that states a larger capacity than the plan has, with more rows than it has records for."""
+    c = Case(40, 6, 512, 512, 16, "fp16", dense=True, seed=8)
+    small = L.LoraPlan(2, 6).build(c.ids_dev[:2].contiguous(), L.adapters_of(c.pool))
+    small.max_tokens = 64                                     # what the caller claims
+    ws = L.LoraWorkspace(64, 1, 512)
+    y = torch.zeros(40, 512, dtype=torch.float16, device="cuda")
+    assert raw_apply([(c.x, y, c.pool)], small, 0, ws, 40, _lib.NO_TENSOR) == 0
+    torch.cuda.synchronize()
+    assert not y.any()
+    with pytest.raises(L.LoraError) as e:
+        ws.check()
+    assert e.value.code == -2
