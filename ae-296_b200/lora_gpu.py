@@ -111,7 +111,7 @@ class Lora_GPU:
     # of three each) and the k and v calls hand out their parts; a k or v call that does not follow
     # such a q call computes its own.
     def _fused_key(self, x, layer_id, prefill):
-        return (x.data_ptr(), x._version, tuple(x.shape), int(layer_id), bool(prefill))
+        return (x.data_ptr(), x._version, x.shape, int(layer_id), bool(prefill))
 
     def _invoke(self, which, x, layer_id, prefill):
         key = self._fused_key(x, layer_id, prefill)
