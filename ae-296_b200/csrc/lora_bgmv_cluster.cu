@@ -372,6 +372,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
         live = false;
     }
     if (!live) {
+        __syncwarp();                                      // the cluster barrier is for whole warps
         cluster_wait();                                    // pairs with the arrival above
         pdl_wait_prior();
         if (tid == 0) pdl_launch_dependents();
