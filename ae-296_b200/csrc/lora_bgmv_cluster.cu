@@ -366,8 +366,9 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     // the same decision in all CTAs of the cluster
     bool live = !hdr.error && seg < hdr.n_wsegs && heads;
     const bool rank_ok = (u.rank == 8 || u.rank == 16 || u.rank == 32 || u.rank == 64) && u.rank <= p.r_cap;
-    const bool mismatch = !hdr.error && (hdr.cap != p.cap || hdr.n_tokens != p.n_tokens || (live && !rank_ok));
-    if (mismatch) {
+    const bool refused = hdr.error || hdr.cap != p.cap || hdr.n_tokens != p.n_tokens;      // the whole plan
+    const bool bad_rank = !refused && live && !rank_ok;                                    // this segment
+    if ((refused && !hdr.error) || bad_rank) {
         if (tid == 0) atomicMax(err, kErrPlanMismatch);
         live = false;
     }
@@ -376,12 +377,18 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
         cluster_wait();                                    // pairs with the arrival above
         pdl_wait_prior();
         if (tid == 0) pdl_launch_dependents();
-        // nothing applies: the clusters are as many as rows times projections, and each clears its row
-        if ((p.flags & B200_LORA_OVERWRITE) && (hdr.error || mismatch)) {
+        // What nothing is applied to is cleared: the rows of the segment, or of a refused plan all rows (the
+        // clusters are as many as rows times projections, and each clears one).
+        if ((p.flags & B200_LORA_OVERWRITE) && (refused || bad_rank)) {
             const ProjArgs& pj = p.proj[item - seg * p.n_proj];
             const int es = p.y_f32 ? 4 : 2;
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<char*>(pj.y) + (long long)seg * pj.ldy * es);
-            for (int q = (int)crank * kThreads + tid; q < pj.h_out * es / 16; q += kCluster * kThreads) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (refused ? i > 0 : i >= u.ntok) break;
+                const int row = refused ? seg : u.tok[i];
+                uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<char*>(pj.y) + (long long)row * pj.ldy * es);
+                for (int q = (int)crank * kThreads + tid; q < pj.h_out * es / 16; q += kCluster * kThreads) dst[q] = make_uint4(0u, 0u, 0u, 0u);
+            }
         }
         return;
     }

@@ -336,3 +336,22 @@ def test_overwrite_equals_accumulating_into_zeros(kind, y_dtype):
     torch.cuda.synchronize()
     assert bool((got == 0).all())
     assert bool(torch.isnan(big[0]).all()) and bool(torch.isnan(big[:, 8 + h:]).all())
+
+
+def test_overwrite_clears_the_rows_of_a_segment_that_does_not_fit():
+    """A segment whose rank is above what the call's table says is not applied and the call says so: exactly that
+    segment's rows are zeros, the others hold their delta."""
+    ids = np.array([1, 0, 1, 0, 0], np.int32)
+    c = Case(5, 2, 512, 512, np.array([8, 64], np.int32), "fp16", seed=12, ids=ids, n_layers=1)
+    want = c.run(0)
+    batch = L.LoraBatch(5, 2, 512, 1).set_ids(c.ids_dev, c.pool)
+    table = L.adapters_of(c.pool)
+    table.r_pool = 8
+    y = torch.full((5, 512), 3.0, dtype=torch.float16, device="cuda")
+    L.apply([(c.x, y, c.pool)], batch.plan, 0, batch.workspace, _lib.NO_TENSOR | _lib.OVERWRITE, table)
+    torch.cuda.synchronize()
+    with pytest.raises(L.LoraError) as e:
+        batch.workspace.check()
+    assert e.value.code == -2
+    rows = torch.from_numpy(ids == 0).cuda()
+    assert torch.equal(y[rows], want[rows]) and not y[~rows].any()
