@@ -35,7 +35,7 @@ def plan_for_requests(batch: LoraBatch, pool: AdapterPool, lora_ids: torch.Tenso
     Prefill: the rows of request ``b`` are ``[b_start_loc[b], b_start_loc[b] + b_seq_len[b])`` of the un-padded
     token matrix, so every request is one segment of adapter ``lora_ids[b]`` and long prompts go to the
     tensor-core tiles.  Decode: one row per request, ``lora_ids`` is the per-token id vector itself.
-    All three are int32 CUDA tensors, as the reference makes them."""
+    All three are int32 CUDA tensors, as the reference makes them (``b_start_loc`` may be on the host)."""
     if lora_ids.dtype != torch.int32 or b_start_loc.dtype != torch.int32 or b_seq_len.dtype != torch.int32:
         raise ValueError("lora_ids, b_start_loc and b_seq_len are int32 tensors")
     n_req = lora_ids.numel()
@@ -47,7 +47,7 @@ def plan_for_requests(batch: LoraBatch, pool: AdapterPool, lora_ids: torch.Tenso
         return batch.set_ids(lora_ids.contiguous(), pool, tiles=False)
     # the library takes the start of every request and ends the last one at total_token_num: building a table
     # with the end in it took a small copy from the host, which waits for everything queued before it
-    return batch.set_segments(b_start_loc.contiguous(), lora_ids.contiguous(), int(total_token_num), pool, tiles=True)
+    return batch.set_segments(b_start_loc.to(lora_ids.device).contiguous(), lora_ids.contiguous(), int(total_token_num), pool, tiles=True)
 
 
 def delta_cost_us(ranks_of_requests: Sequence[int], tokens_of_requests: Sequence[int], adapters_of_requests: Sequence[int],

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import ae296_b200 as L
+from ae296_b200.batching import plan_for_requests
 from lora_testlib import TOL, Case, rel_err
 from oracle import lora_oracle as O
 
@@ -259,3 +260,17 @@ np.save(sys.argv[1], y.float().cpu().numpy())
         subprocess.run([sys.executable, "-c", script, path], check=True, env=env, timeout=300)
         outs.append(np.load(path))
     assert np.abs(outs[0]).max() > 0 and np.array_equal(outs[0], outs[1])
+
+
+def test_plan_for_requests_takes_start_rows_on_the_host():
+    lens, owner = [40, 3, 70], [2, 0, 1]
+    c = seg_case(lens, owner, [16, 32, 64], 3, 256, 256, "fp16", seed=5)
+    starts = torch.from_numpy(np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int32))
+    ids, seq = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (owner, lens))
+    ys = []
+    for where in ("cuda", "cpu"):
+        batch = L.LoraBatch(c.T, 3, 256, 1)
+        plan_for_requests(batch, c.pool, ids, starts.to(where), seq, c.T, prefill=True)
+        ys.append(torch.zeros(c.T, 256, dtype=torch.float16, device="cuda"))
+        batch.apply([(c.x, ys[-1], c.pool)], 0)
+    assert ys[0].any() and torch.equal(ys[0], ys[1])
