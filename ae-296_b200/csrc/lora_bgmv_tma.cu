@@ -32,8 +32,8 @@
 // expand: the first unit a CTA has of a segment brings the intermediate along: its producer
 // adds up the segment's slots in ascending k order (bit-reproducible) straight into the stage.
 // The weight tile is the MMA's A operand (16 output columns x 16 rank indices), the N columns
-// hold the hi and lo 16-bit halves of four tokens' fp32 intermediate, so one MMA is exact for
-// four tokens; results are added into the staged y tile, which each warp writes back itself.
+// hold the hi and lo 16-bit halves of four tokens' fp32 intermediate (together it to 2^-17 in bf16, 2^-23 or
+// 2^-25 absolute in fp16), so one MMA serves four tokens; results are added into the staged y tile, which each warp writes back itself.
 //
 // PAD: a dense pool [N, L, R, h_in] / [N, L, h_out, R] whose adapters have any rank r <= R.  An
 // adapter is worked on as its rank class 8 / 16 / 32 / 64 (the next one up), with the units, slots

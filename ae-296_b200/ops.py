@@ -253,8 +253,8 @@ def add_lora_bgmv(y: torch.Tensor, x: torch.Tensor, wa_T_all: torch.Tensor, wb_T
     ``wa_T_all [N, L, r, h_in]``, ``wb_T_all [N, L, h_out, r]`` contiguous fp16/bf16 CUDA
     tensors, ``indicies [T]`` int64 (or int32) CUDA tensor.  Returns ``None``.
 
-    Two launches (shrink, expand) when the index tensor is the one of the previous call on this
-    stream, unmodified; one more (the plan kernel) when it is new.
+    One launch for a few tokens (a cluster per token, as many as run at once), else two (shrink, expand), when
+    the index tensor is the one of the previous call on this stream, unmodified; one more (the plan kernel) when it is new.
     """
     rc = _lib.host().bgmv(y, x, wa_T_all, wb_T_all, indicies, layer_idx, scale)
     if rc <= 0:
