@@ -418,8 +418,8 @@ PyObject* py_bgmv_static(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return PyLong_FromLong(rc);
 }
 
-// stream_key(tensor) -> (current stream of the tensor's device, identifier of the capture it is in or 0)
-PyObject* py_stream_key(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+// (current stream of the tensor's device, identifier of the capture it is in or 0)
+PyObject* stream_and_capture(PyObject* const* args, Py_ssize_t nargs) {
     if (nargs != 1 || !THPVariable_Check(args[0]) || !THPVariable_Unpack(args[0]).is_cuda()) {
         PyErr_SetString(PyExc_ValueError, "a CUDA tensor expected");
         return nullptr;
@@ -433,6 +433,30 @@ PyObject* py_stream_key(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
     return Py_BuildValue("(KK)", reinterpret_cast<unsigned long long>(stream), cap);
 }
+// stream_key(tensor) -> (stream, capture)
+PyObject* py_stream_key(PyObject*, PyObject* const* args, Py_ssize_t nargs) { return stream_and_capture(args, nargs); }
+
+// use_key(tensor) -> ((stream, capture), address, version, *sizes, *strides): equal for two uses of the same values in one place
+PyObject* py_use_key(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    Ref where(stream_and_capture(args, nargs));
+    if (!where) return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(args[0]);
+    const unsigned long long ptr = reinterpret_cast<uintptr_t>(t.data_ptr());
+    const unsigned long version = t._version();                     // (throws for an inference tensor)
+    const int64_t dim = t.dim();
+    Ref key(PyTuple_New(3 + 2 * dim));
+    if (!key) return nullptr;
+    Py_INCREF(where.o);
+    PyTuple_SET_ITEM(key.o, 0, where.o);
+    for (int64_t i = 0; i < 2 + 2 * dim; ++i) {
+        PyObject* v = i == 0 ? PyLong_FromUnsignedLongLong(ptr) : i == 1 ? PyLong_FromUnsignedLong(version)
+                      : PyLong_FromLongLong(i < 2 + dim ? t.size(i - 2) : t.stride(i - 2 - dim));
+        if (!v) return nullptr;
+        PyTuple_SET_ITEM(key.o, 1 + i, v);
+    }
+    Py_INCREF(key.o);
+    return key.o;
+}
 
 PyMethodDef kMethods[] = {
     {"apply", (PyCFunction)(void*)guarded<py_apply>, METH_FASTCALL, nullptr},
@@ -441,6 +465,7 @@ PyMethodDef kMethods[] = {
     {"bgmv", (PyCFunction)(void*)guarded<py_bgmv>, METH_FASTCALL, nullptr},
     {"bgmv_static", (PyCFunction)(void*)guarded<py_bgmv_static>, METH_FASTCALL, nullptr},
     {"stream_key", (PyCFunction)(void*)guarded<py_stream_key>, METH_FASTCALL, nullptr},
+    {"use_key", (PyCFunction)(void*)guarded<py_use_key>, METH_FASTCALL, nullptr},
     {"bgmv_register", py_bgmv_register, METH_VARARGS, nullptr},
     {"bgmv_forget", (PyCFunction)(void*)guarded<py_bgmv_forget>, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

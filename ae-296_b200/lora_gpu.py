@@ -81,9 +81,9 @@ class Lora_GPU:
         # Plan + workspace per (decode batch size, or None for prefill; stream; graph capture or 0), so that a
         # step on another stream, and every replay of a graph, which builds its plan again, leaves this one's alone.
         self._kept = {}
-        self._stream_key = _lib.host().stream_key
+        self._use_key = _lib.host().use_key
         self._indices_version = {}       # decode batch size -> how often set_indices has set it
-        self._fused = None               # (x identity, layer, prefill) -> the k and v deltas computed with q
+        self._fused = None               # (use of x, layer, prefill) -> the k and v deltas computed with q
 
     def set_indices(self, indices: torch.Tensor) -> None:
         """Adapter slot of each decode token for batches of ``len(indices)`` tokens.  A captured graph goes on
@@ -91,12 +91,11 @@ class Lora_GPU:
         bsz = indices.numel()
         self.select_inds[bsz - 1] = indices.to(device=f"cuda:{self.device}")
         self._indices_version[bsz] = self._indices_version.get(bsz, 0) + 1
+        self._fused = None
 
-    def _keep(self, x, kind, rows, n_adapters) -> _Kept:
-        """What is kept for calls of ``kind`` on the stream (and in the capture) that ``x`` is used on, with room
-        for ``rows``.  A capture's is allocated inside it, so its memory belongs to the graph's pool; the
+    def _keep(self, x, where, kind, rows, n_adapters) -> _Kept:
+        """What is kept for calls of ``kind`` on the stream and in the capture ``where``, with room for ``rows``.  A capture's is allocated inside it, so its memory belongs to the graph's pool; the
         reference here goes when the stream, which is in one capture at a time, makes its next."""
-        where = self._stream_key(x)
         kept = self._kept.get((kind, where))
         if kept is None or kept.rows < rows:
             for key in [k for k in self._kept if k[1][0] == where[0] and k[1][1] not in (0, where[1])]:
@@ -109,19 +108,17 @@ class Lora_GPU:
     # (lightllm/models/llama/layer_infer/transformer_layer_infer.py:108-111).  The q call computes
     # all three deltas in one fused pass (x is read once, one shrink and one expand launch instead
     # of three each) and the k and v calls hand out their parts; a k or v call that does not follow
-    # such a q call computes its own.
-    def _fused_key(self, x, layer_id, prefill):
-        return (x.data_ptr(), x._version, x.shape, int(layer_id), bool(prefill))
-
+    # such a q call, on the same stream and in the same graph capture, computes its own.
     def _invoke(self, which, x, layer_id, prefill):
-        key = self._fused_key(x, layer_id, prefill)
+        use = self._use_key(x)
+        key = (use, int(layer_id), bool(prefill))
         if which > 0 and self._fused is not None and self._fused[0] == key:
             out = self._fused[1][which]
             if which == 2:
                 self._fused = None
             return out
         projs = (0, 1, 2) if which == 0 else (which,)
-        ys = self._prefill(x, layer_id, projs) if prefill else self._decode(x, layer_id, projs)
+        ys = (self._prefill if prefill else self._decode)(x, use[0], layer_id, projs)
         if which == 0:
             self._fused = (key, ys)
         return ys[which]
@@ -135,10 +132,10 @@ class Lora_GPU:
     def invoke_one_layer_v(self, x, layer_id, prefill=False):
         return self._invoke(2, x, layer_id, prefill)
 
-    def _decode(self, x, layer_id, projs):
+    def _decode(self, x, where, layer_id, projs):
         """x ``[bsz, H]``; token ``t`` uses slot ``select_inds[bsz-1][t]`` (lora_gpu.py:137-138)."""
         bsz = x.shape[0]
-        kept = self._keep(x, bsz, bsz, self.batch_size)
+        kept = self._keep(x, where, bsz, bsz, self.batch_size)
         batch = kept.batch
         version = self._indices_version.get(bsz, 0)
         if kept.built != version:
@@ -149,13 +146,13 @@ class Lora_GPU:
               _lib.NO_TENSOR | _lib.OVERWRITE, self._ad_decode)
         return y                         # only those of `projs` hold anything
 
-    def _prefill(self, x, layer_id, projs):
+    def _prefill(self, x, where, layer_id, projs):
         """x ``[B, L, H]``: request ``b`` uses prefill slot ``b`` (lora_gpu.py:125-128).  One plan +
         workspace (per stream) serves every shape: it grows to the largest batch seen and the segment table is
         rebuilt (one small kernel) when ``(B, L)`` changes, so nothing accumulates per shape."""
         bsz, seqlen, hidden = x.shape
         rows = bsz * seqlen
-        kept = self._keep(x, None, rows, self.max_prefill_batch_size)
+        kept = self._keep(x, where, None, rows, self.max_prefill_batch_size)
         batch = kept.batch
         if kept.built != (bsz, seqlen):
             starts = torch.arange(0, (bsz + 1) * seqlen, seqlen, dtype=torch.int32, device=x.device)

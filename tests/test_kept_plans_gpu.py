@@ -223,3 +223,40 @@ def test_layer_object_prefill_shape_only_captured():
         rms = float(want.pow(2).mean().sqrt())
         # one rounding of the result, and of an intermediate that may fall on the other side of a tie
         assert float((got[i].float() - want).abs().max()) <= 2e-3 * rms + float(want.abs().max()) * 2 ** -10
+
+
+def test_layer_object_parts_of_a_captured_or_foreign_q_call_are_not_handed_out():
+    """k after a q call that was only captured, or that ran on another stream: its own computation."""
+    obj, x, (a, _), _ = _layer_object()
+    obj.set_indices(a)
+    want = obj.invoke_one_layer_k(x, 1).clone()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        obj.invoke_one_layer_q(x, 0)                       # warm-up
+        part = {}
+
+        def q():
+            obj.invoke_one_layer_q(x, 1)
+            part["k"] = obj._fused[1][1]
+
+        g = _capture(s, q)
+        k = obj.invoke_one_layer_k(x, 1)
+    torch.cuda.synchronize()
+    assert k.data_ptr() != part["k"].data_ptr() and torch.equal(k, want)
+    obj.invoke_one_layer_q(x, 1)
+    other = obj._fused[1][1]
+    with torch.cuda.stream(s):
+        k = obj.invoke_one_layer_k(x, 1)
+    torch.cuda.synchronize()
+    assert k.data_ptr() != other.data_ptr() and torch.equal(k, want)
+
+
+def test_layer_object_parts_of_a_q_call_with_other_indices_are_not_handed_out():
+    obj, x, (a, b), _ = _layer_object()
+    obj.set_indices(b)
+    want = obj.invoke_one_layer_k(x, 1).clone()
+    obj.set_indices(a)
+    obj.invoke_one_layer_q(x, 1)
+    obj.set_indices(b)
+    assert torch.equal(obj.invoke_one_layer_k(x, 1), want)
