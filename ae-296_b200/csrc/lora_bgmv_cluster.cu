@@ -63,13 +63,13 @@ struct ClusterArgs {
 struct Layout {
     int pitch, x, b, y, ypitch, red, vs, vt, bars, total;
 };
-__host__ __device__ inline Layout layout_of(int r_cap, int kcols, int jcols) {
+__host__ __device__ inline Layout layout_of(int r_cap, int kcols, int jcols, int y_f32) {
     Layout l;
     l.pitch = kcols * 2 + 64;                              // A and x rows
     l.x = r_cap * l.pitch;
     l.b = l.x + 8 * l.pitch;
     l.y = l.b + jcols * r_cap * 2;
-    l.ypitch = jcols * 2 + 32;
+    l.ypitch = jcols * (y_f32 ? 4 : 2) + 32;
     l.red = l.y + 8 * l.ypitch;
     l.vs = l.red + kRedBytes;                              // cross-warp reduction: [slice][token][rank]
     l.vt = l.vs + kCluster * 8 * r_cap * 4;                // the eight partials: [cta][token][rank]
@@ -250,10 +250,9 @@ __device__ __forceinline__ void cluster_expand(const ClusterArgs& p, const ProjA
             if (row[grp] >= 0) {
             const long long yoff = (long long)row[grp] * pj.ldy + j0 + jl;
             if (p.y_f32) {
-                float2* yp = reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff);
-                float2 yv = overwrite ? make_float2(0.f, 0.f) : *yp;
+                float2 yv = overwrite ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(ysm + (t + 4 * grp) * ypitch + jl * 4);
                 yv.x += d0; yv.y += d1;
-                *yp = yv;
+                *reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff) = yv;
             } else {
                 const unsigned yw = overwrite ? 0u : *reinterpret_cast<const unsigned*>(ysm + (t + 4 * grp) * ypitch + jl * 2);
                 float lo, hi;
@@ -330,7 +329,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     const unsigned crank = cluster_rank();
     const int item = blockIdx.x / kCluster, seg = item / p.n_proj;      // seg < n_tokens <= cap
     cluster_arrive();
-    const Layout l = layout_of(p.r_cap, p.kcols, p.jcols);
+    const Layout l = layout_of(p.r_cap, p.kcols, p.jcols, p.y_f32);
     PlanView pv = plan_view(p.plan, p.cap, p.n_adapters);
     unsigned* err = &reinterpret_cast<WorkspaceCtl*>(p.workspace)->error;
     // header and segment record in one round trip (the record of a segment the plan does not have is not used; it is
@@ -416,7 +415,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
     pdl_wait_prior();
     if (tid == 0) pdl_launch_dependents();
     if (warp == 1) {
-        const int y_bytes = p.y_f32 || (p.flags & B200_LORA_OVERWRITE) ? 0 : njs * 2;
+        const int y_size = p.y_f32 ? 4 : 2;
+        const int y_bytes = p.flags & B200_LORA_OVERWRITE ? 0 : njs * y_size;
         if (lane == 0) { mbar_arrive_expect_tx(bar_a, u.ntok * ncol * 2); mbar_arrive_expect_tx(bar_b, u.ntok * y_bytes); }
         __syncwarp();
         const int q = lane & 7;
@@ -428,7 +428,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) bgm
             if (lane < 8 && ncol > 0)
                 bulk_g2s(sbase + l.x + q * l.pitch, reinterpret_cast<const T*>(pj.x) + (long long)tok * pj.ldx + k0, ncol * 2, bar_a);
             else if (lane >= 8 && lane < 16 && y_bytes > 0)
-                bulk_g2s(sbase + l.y + q * l.ypitch, reinterpret_cast<const T*>(pj.y) + (long long)tok * pj.ldy + j0, y_bytes, bar_b);
+                bulk_g2s(sbase + l.y + q * l.ypitch, reinterpret_cast<const char*>(pj.y) + ((long long)tok * pj.ldy + j0) * y_size, y_bytes, bar_b);
         }
         __syncwarp();
     }
@@ -485,7 +485,7 @@ bool bgmv_cluster_fits(const ApplyParams& p) {
         if (widest_slice(p.proj[i].h_out) > jcols) jcols = widest_slice(p.proj[i].h_out);
     }
     if (kcols > 1024 || jcols > 1024) return false;
-    const int smem = layout_of(pad_rank(p.r_pool), kcols, jcols).total;
+    const int smem = layout_of(pad_rank(p.r_pool), kcols, jcols, p.y_f32).total;
     return smem <= kMaxSmem;
 }
 
@@ -495,7 +495,7 @@ int bgmv_cluster_limit(const ApplyParams& p, int io_dtype) {
         if (widest_slice(p.proj[i].h_in) > kcols) kcols = widest_slice(p.proj[i].h_in);
         if (widest_slice(p.proj[i].h_out) > jcols) jcols = widest_slice(p.proj[i].h_out);
     }
-    const int smem = layout_of(pad_rank(p.r_pool), kcols, jcols).total;
+    const int smem = layout_of(pad_rank(p.r_pool), kcols, jcols, p.y_f32).total;
     return io_dtype == B200_LORA_F16 ? resident_clusters<__half>(smem) : resident_clusters<__nv_bfloat16>(smem);
 }
 
@@ -511,7 +511,7 @@ cudaError_t launch_bgmv_cluster(const ApplyParams& p, const void* ids, int ids_i
     a.plan = p.plan; a.workspace = p.workspace;
     a.n_proj = p.n_proj; a.n_adapters = p.n_adapters; a.n_layers = p.n_layers; a.r_pool = p.r_pool; a.packed = p.packed;
     a.layer = p.layer; a.flags = p.flags; a.y_f32 = p.y_f32; a.cap = p.cap; a.n_tokens = p.n_tokens;
-    const int smem = layout_of(a.r_cap, a.kcols, a.jcols).total;
+    const int smem = layout_of(a.r_cap, a.kcols, a.jcols, a.y_f32).total;
     // a cluster per (work segment, projection); there are at most as many segments as tokens
     const int n = p.n_tokens * p.n_proj;
     a.ids = ids; a.ids_i64 = ids_i64; a.scale = p.scale;
