@@ -39,8 +39,9 @@
 // adapter is worked on as its rank class 8 / 16 / 32 / 64 (the next one up), with the units, slots
 // and MMA shapes of that class.  Its B rows lie R apart, so the weight tile of an expand unit comes
 // as [128 rows x class] boxes of a 2-D map over the B pool, which pack into the same shared-memory
-// layout as a contiguous block; the map promotes nothing in L2, so a row costs the sectors of its
-// class and not all R columns.  What lies between r and the class is not part of the adapter and may
+// layout as a contiguous block.  DRAM is read in full 128-byte lines all the same, though the map promotes
+// nothing in L2: at R = 64 every row costs all of its columns (40.4 MB a q/k/v launch of the step below, 25 at the
+// classes).  What lies between r and the class is not part of the adapter and may
 // hold anything: those rows of the intermediate are written as zeros when a run is flushed, and those
 // columns of the weight fragments are masked out in registers (a product with zero would let a NaN
 // through).  A 93-token decode step, ranks 8 to 64 in
