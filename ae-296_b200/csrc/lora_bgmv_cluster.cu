@@ -174,16 +174,97 @@ __device__ __forceinline__ void cluster_fold(const float* vs, float* vt, int nto
 
 // The weight tile is the MMA's A operand: 16 output columns (M) by 16 rank indices (K, permuted so
 // that a thread's fragments are wide loads).  Column 2q of N holds the hi half of token q's
-// intermediate and column 2q+1 the lo half (tokens 0..3, then 4..7 with a second MMA); thread (g, t)
+// intermediate and column 2q+1 the lo half (tokens 0..3, then 4..7 with a second MMA: NG groups); thread (g, t)
 // gets token t's products for columns g and g + 8, and lanes g and g ^ 1 swap one so that each owns two
 // adjacent outputs.
+//
+// What bounds it: two warps a scheduler do not hide the chain of an MMA group (four dependent MMAs at rank 64, the
+// swap, the store), so a warp works on two blocks of columns and both groups of tokens at once, with nothing but
+// independent chains between the loads and the stores.  Five tokens of one adapter, 1024 to 8192 columns, rank 64, where
+// a CTA has most to do: 6.6 us with a block at a time, 5.65 now (two kernels: 5.8); 4096 columns, rank 16: 3.5 and 3.2 (5.0).
+template <typename T, int R, int NG>
+__device__ __forceinline__ void expand_columns(const ClusterArgs& p, const ProjArgs& pj, float scale, const unsigned (&bf)[2][R == 64 ? 4 : R == 32 ? 2 : 1][2],
+                                               const int (&row)[2], const unsigned char* b, const unsigned char* ysm, int ypitch, int j0,
+                                               int njs, int lane, int warp) {
+    constexpr int KS = R == 64 ? 4 : R == 32 ? 2 : 1;
+    constexpr int kStep = kWarps * 16;
+    const int g = lane >> 2, t = lane & 3;
+    const bool overwrite = (p.flags & B200_LORA_OVERWRITE) != 0;      // y counts as zero
+    const bool lo_half = (g & 1) != 0;
+    for (int nb0 = warp * 16; nb0 < njs; nb0 += 2 * kStep) {
+        const bool two = nb0 + kStep < njs;                // else the second block repeats the first and stores nothing
+        unsigned a[2][KS][4];
+        float acc[2][NG][4];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int nb = i == 1 && two ? nb0 + kStep : nb0;
+            const unsigned char* w0 = b + (nb + g) * (R * 2);      // output column g of the block
+            const unsigned char* w1 = w0 + 8 * (R * 2);            // output column g + 8
+            if constexpr (R >= 32) {
+#pragma unroll
+                for (int c = 0; c < KS / 2; ++c) {
+                    const uint4 r0 = *reinterpret_cast<const uint4*>(w0 + (t * (KS / 2) + c) * 16);
+                    const uint4 r1 = *reinterpret_cast<const uint4*>(w1 + (t * (KS / 2) + c) * 16);
+                    a[i][2 * c][0] = r0.x; a[i][2 * c][1] = r1.x; a[i][2 * c][2] = r0.y; a[i][2 * c][3] = r1.y;
+                    a[i][2 * c + 1][0] = r0.z; a[i][2 * c + 1][1] = r1.z; a[i][2 * c + 1][2] = r0.w; a[i][2 * c + 1][3] = r1.w;
+                }
+            } else if constexpr (R == 16) {
+                const uint2 r0 = *reinterpret_cast<const uint2*>(w0 + t * 8);
+                const uint2 r1 = *reinterpret_cast<const uint2*>(w1 + t * 8);
+                a[i][0][0] = r0.x; a[i][0][1] = r1.x; a[i][0][2] = r0.y; a[i][0][3] = r1.y;
+            } else {
+                a[i][0][0] = *reinterpret_cast<const unsigned*>(w0 + t * 4);
+                a[i][0][1] = *reinterpret_cast<const unsigned*>(w1 + t * 4);
+                a[i][0][2] = a[i][0][3] = 0u;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int grp = 0; grp < NG; ++grp) acc[i][grp][0] = acc[i][grp][1] = acc[i][grp][2] = acc[i][grp][3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int grp = 0; grp < NG; ++grp)
+                    Mma<T>::run(acc[i][grp], a[i][k][0], a[i][k][1], a[i][k][2], a[i][k][3], bf[grp][k][0], bf[grp][k][1]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int jl = nb0 + i * kStep + (lo_half ? g + 7 : g);
+#pragma unroll
+            for (int grp = 0; grp < NG; ++grp) {
+                const float c_lo = scale * (acc[i][grp][0] + acc[i][grp][1]);
+                const float c_hi = scale * (acc[i][grp][2] + acc[i][grp][3]);
+                const float got = __shfl_xor_sync(0xffffffffu, lo_half ? c_lo : c_hi, 4);
+                const float d0 = lo_half ? got : c_lo, d1 = lo_half ? c_hi : got;
+                if (row[grp] < 0 || (i == 1 && !two)) continue;
+                const long long yoff = (long long)row[grp] * pj.ldy + j0 + jl;
+                if (p.y_f32) {
+                    float2 yv = overwrite ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(ysm + (t + 4 * grp) * ypitch + jl * 4);
+                    yv.x += d0; yv.y += d1;
+                    *reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff) = yv;
+                } else {
+                    const unsigned yw = overwrite ? 0u : *reinterpret_cast<const unsigned*>(ysm + (t + 4 * grp) * ypitch + jl * 2);
+                    float lo, hi;
+                    if (Cvt<T>::is_bf16) {
+                        lo = __uint_as_float(yw << 16); hi = __uint_as_float(yw & 0xffff0000u);
+                    } else {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&yw));
+                        lo = f.x; hi = f.y;
+                    }
+                    *reinterpret_cast<unsigned*>(reinterpret_cast<T*>(pj.y) + yoff) = Cvt<T>::pack2(lo + d0, hi + d1);
+                }
+            }
+        }
+    }
+}
+
 template <typename T, int R>
 __device__ __forceinline__ void cluster_expand(const ClusterArgs& p, const ProjArgs& pj, const UnitRec& u, const unsigned char* b,
                                                const unsigned char* ysm, int ypitch, const float* vt, int j0, int njs, int lane, int warp) {
     constexpr int KS = R == 64 ? 4 : R == 32 ? 2 : 1;
     const int g = lane >> 2, t = lane & 3;
-    const int ngrp = u.ntok > 4 ? 2 : 1;
-    const bool overwrite = (p.flags & B200_LORA_OVERWRITE) != 0;      // y counts as zero
     const bool lo_half = (g & 1) != 0;
     unsigned bf[2][KS][2];
 #pragma unroll
@@ -214,59 +295,9 @@ __device__ __forceinline__ void cluster_expand(const ClusterArgs& p, const ProjA
         for (int i = 1; i < 8; ++i)
             if (q == i && q < u.ntok) row[grp] = u.tok[i];
     }
-#pragma unroll 2
-    for (int nb = warp * 16; nb < njs; nb += kWarps * 16) {
-        const unsigned char* w0 = b + (nb + g) * (R * 2);      // output column g of the block
-        const unsigned char* w1 = w0 + 8 * (R * 2);            // output column g + 8
-        unsigned a[KS][4];
-        if constexpr (R >= 32) {
-#pragma unroll
-            for (int c = 0; c < KS / 2; ++c) {
-                const uint4 r0 = *reinterpret_cast<const uint4*>(w0 + (t * (KS / 2) + c) * 16);
-                const uint4 r1 = *reinterpret_cast<const uint4*>(w1 + (t * (KS / 2) + c) * 16);
-                a[2 * c][0] = r0.x; a[2 * c][1] = r1.x; a[2 * c][2] = r0.y; a[2 * c][3] = r1.y;
-                a[2 * c + 1][0] = r0.z; a[2 * c + 1][1] = r1.z; a[2 * c + 1][2] = r0.w; a[2 * c + 1][3] = r1.w;
-            }
-        } else if constexpr (R == 16) {
-            const uint2 r0 = *reinterpret_cast<const uint2*>(w0 + t * 8);
-            const uint2 r1 = *reinterpret_cast<const uint2*>(w1 + t * 8);
-            a[0][0] = r0.x; a[0][1] = r1.x; a[0][2] = r0.y; a[0][3] = r1.y;
-        } else {
-            a[0][0] = *reinterpret_cast<const unsigned*>(w0 + t * 4);
-            a[0][1] = *reinterpret_cast<const unsigned*>(w1 + t * 4);
-            a[0][2] = a[0][3] = 0u;
-        }
-        const int jl = nb + (lo_half ? g + 7 : g);
-#pragma unroll
-        for (int grp = 0; grp < 2; ++grp) {
-            if (grp >= ngrp) break;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int k = 0; k < KS; ++k) Mma<T>::run(acc, a[k][0], a[k][1], a[k][2], a[k][3], bf[grp][k][0], bf[grp][k][1]);
-            const float c_lo = u.scale * (acc[0] + acc[1]);
-            const float c_hi = u.scale * (acc[2] + acc[3]);
-            const float got = __shfl_xor_sync(0xffffffffu, lo_half ? c_lo : c_hi, 4);
-            const float d0 = lo_half ? got : c_lo, d1 = lo_half ? c_hi : got;
-            if (row[grp] >= 0) {
-            const long long yoff = (long long)row[grp] * pj.ldy + j0 + jl;
-            if (p.y_f32) {
-                float2 yv = overwrite ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(ysm + (t + 4 * grp) * ypitch + jl * 4);
-                yv.x += d0; yv.y += d1;
-                *reinterpret_cast<float2*>(reinterpret_cast<float*>(pj.y) + yoff) = yv;
-            } else {
-                const unsigned yw = overwrite ? 0u : *reinterpret_cast<const unsigned*>(ysm + (t + 4 * grp) * ypitch + jl * 2);
-                float lo, hi;
-                if (Cvt<T>::is_bf16) {
-                    lo = __uint_as_float(yw << 16); hi = __uint_as_float(yw & 0xffff0000u);
-                } else {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&yw));
-                    lo = f.x; hi = f.y;
-                }
-                *reinterpret_cast<unsigned*>(reinterpret_cast<T*>(pj.y) + yoff) = Cvt<T>::pack2(lo + d0, hi + d1);
-            }
-            }
-        }
-    }
+    __syncwarp();                                          // the MMAs are for whole warps
+    if (u.ntok > 4) expand_columns<T, R, 2>(p, pj, u.scale, bf, row, b, ysm, ypitch, j0, njs, lane, warp);
+    else expand_columns<T, R, 1>(p, pj, u.scale, bf, row, b, ysm, ypitch, j0, njs, lane, warp);
 }
 
 template <typename T, int R>

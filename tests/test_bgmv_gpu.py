@@ -48,7 +48,7 @@ def test_dense_pool_ranks_not_multiple_of_8_and_garbage_padding():
     assert rel_err(y32.double().cpu().numpy(), c.oracle_delta(0)) <= TOL
 
 
-@pytest.mark.parametrize("h_in,h_out", [(128, 128), (640, 1152), (1152, 640), (2048, 8192), (8192, 1024)])
+@pytest.mark.parametrize("h_in,h_out", [(128, 128), (640, 1152), (1152, 640), (256, 3072), (2048, 8192), (8192, 1024)])
 @pytest.mark.parametrize("T,N,ranks,dtype", [(1, 1, [64], "bf16"), (8, 1, [8], "fp16"), (5, 2, [32, 16], "bf16"), (10, 4, [8, 64, 16, 32], "fp16")])
 def test_few_tokens_in_one_launch(T, N, ranks, dtype, h_in, h_out):
     """The cluster kernel: every rank, one to eight tokens a segment, slices of h_in and h_out that are empty or
