@@ -165,12 +165,13 @@ bool fast_ranks(const b200_lora_adapters* ad) {
 // second round of clusters would pay the chain again, while the two streaming kernels only get longer.
 // Microseconds per apply, two kernels / cluster kernel, distinct adapters, weights from HBM, graph replay; items =
 // tokens x projections.  bgmv_cluster_limit() is the item count of the last column that is inside the rule:
-//   h 4096, r 16 (3 CTAs an SM):  1 item 5.5 / 2.6   24 items 7.2 / 4.2   46 items 8.5 / 6.3   limit 48: 8.5 / 6.8   beyond, 64: 9.7 / 10.5
-//   h 2048, r 64 (2 CTAs an SM):  1 item 6.1 / 3.9   24 items 8.6 / 6.3   31 items 9.4 / 7.2   limit 33: 9.5 / 8.4   beyond, 36: 10.2 / 11.7
-//   h 4096, r 64 (1 CTA an SM):   1 item 6.8 / 4.4   12 items 9.1 / 6.4   13 items 9.3 / 6.6   limit 15: 9.7 / 6.9   beyond, 16: 10.4 / 11.9
+//   h 4096, r 16 (3 CTAs an SM):  1 item 5.5 / 3.6   24 items 7.2 / 4.2   46 items 8.5 / 6.3   limit 48: 8.5 / 6.8   beyond, 64: 9.7 / 10.5
+//   h 2048, r 64 (2 CTAs an SM):  1 item 6.1 / 4.7   24 items 8.6 / 6.3   31 items 9.4 / 7.2   limit 33: 9.5 / 8.4   beyond, 36: 10.2 / 11.7
+//   h 4096, r 64 (1 CTA an SM):   1 item 6.8 / 5.0   12 items 9.1 / 6.4   13 items 9.3 / 6.6   limit 15: 9.7 / 6.9   beyond, 16: 10.4 / 11.9
 // The limit is the right line at the other sizes too: h 4096, r 32 (33): 9.2 / 8.1; h 8192, r 16 (33): 9.4 / 8.8;
 // h 5120, r 32 (15): 8.2 / 5.6; h 4096 to 1024, r 64 (15): 8.5 / 5.9; three projections, r 16 (48): 8.5 / 6.8; and with
-// few adapters, whose clusters are fewer than the items: 8 tokens of one, h 1024 to 8192, r 64: 5.85 / 5.80; r 16: 5.2 / 4.2.
+// few adapters, whose clusters are fewer than the items (weights in L2): 8 tokens of one, h 1024 to 8192, r 64: 5.85 / 5.80;
+// r 16: 5.2 / 4.2.
 bool cluster_route(const ApplyParams& p, const b200_lora_adapters* ad, int io_dtype) {
     if (p.n_tokens > kClusterTokens) return false;                   // beyond any limit, and what the plan has room for
     const int other = B200_LORA_ONLY_SHRINK | B200_LORA_ONLY_EXPAND | B200_LORA_DELTA_THEN_ADD;

@@ -181,7 +181,8 @@ __device__ __forceinline__ void cluster_fold(const float* vs, float* vt, int nto
 // What bounds it: two warps a scheduler do not hide the chain of an MMA group (four dependent MMAs at rank 64, the
 // swap, the store), so a warp works on two blocks of columns and both groups of tokens at once, with nothing but
 // independent chains between the loads and the stores.  Five tokens of one adapter, 1024 to 8192 columns, rank 64, where
-// a CTA has most to do: 6.6 us with a block at a time, 5.65 now (two kernels: 5.8); 4096 columns, rank 16: 3.5 and 3.2 (5.0).
+// a CTA has most to do, weights in L2: 6.6 us with a block at a time, 5.65 now (two kernels: 5.8); 4096 columns, rank 16:
+// 3.5 and 3.2 (5.0).
 template <typename T, int R, int NG>
 __device__ __forceinline__ void expand_columns(const ClusterArgs& p, const ProjArgs& pj, float scale, const unsigned (&bf)[2][R == 64 ? 4 : R == 32 ? 2 : 1][2],
                                                const int (&row)[2], const unsigned char* b, const unsigned char* ysm, int ypitch, int j0,
